@@ -5,7 +5,7 @@
 // accumulating it.  The layouts:
 //
 //   0  12 x 32-bit limbs: one level of limb Karatsuba (three 6 x 6 products
-//      whose rows are mad.lo.cc / madc.hi.cc carry chains, 216 multiplies)
+//      whose rows are chains of paired mad.lo.cc / madc.hi.cc, 108 pairs)
 //      added into a 26-limb accumulator: the form every verify kernel uses
 //      (fp2ops.cuh prod24k + acc_plus);
 //   1  15 x 26-bit signed limbs: 225 mad.wide.s32 into 29 signed 64-bit
