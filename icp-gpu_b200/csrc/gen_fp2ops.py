@@ -806,6 +806,265 @@ class Emulator:
             slots[d] = v
 
 
+# ---------------------------------------------------------------- paired-warp form
+# The 32-item kernel (verify_w.cu) gives every Fp2 coefficient of an Fp12 result
+# to two warps, one for each component.  An Fp2 product takes three Fp products
+# (Gauss),
+#   X Y = (s - x1 (y0 + y1)) + (s + x0 (y1 - y0)) u,  s = (x0 + x1) y0,
+# of which the first enters the real part alone, the second the imaginary part
+# alone and s both.  So a warp has one accumulator and adds each product to it
+# once: it sums its share of the products that both parts use, stores that partial
+# sum for its partner, goes on to its own part's products, and adds the partner's
+# partial sum before it reduces.  A product's operands are linear forms of one
+# slot, chosen so that products enter with a plus sign:
+#   0, 1   x0, x1                  8       x0 + x1
+#   2, 3   2 x0, 2 x1              9       5p - x0 - x1
+#   4, 5   3p - x0, 3p - x1       10       2 (x0 + x1)
+#   6, 7   x0 - x1 + 3p,          12, 13   2 (3p - x0), 2 (3p - x1)
+#          x1 - x0 + 3p
+# The one exception is xi X^2 = (d - t) + (d + t) u with d = x0^2 - x1^2 and
+# t = 2 x0 x1: t, formed by the imaginary part's warp, is subtracted by the other.
+# A component is
+#   out = QP( scale * REDC(sum of U V) + sum of c_j z_j + bias p ),
+# scale 1 or 3, or 2 (3 REDC + ..) for scale 6 (its linear terms halved); the
+# bias covers the linear terms and the subtracted sum (REDC of a negative sum is
+# a negative thirteen-word value).
+X_0, X_1, X_2X0, X_2X1, X_N0, X_N1, X_D01, X_D10, X_S, X_NS, X_2S = range(11)
+X_2N0, X_2N1 = 12, 13
+X_LINE = 15     # the line coefficient the warp has read from the key's table
+
+
+def form_value(f, x):
+    x0, x1 = x
+    return {X_0: x0, X_1: x1, X_2X0: 2 * x0, X_2X1: 2 * x1, X_N0: K3P - x0, X_N1: K3P - x1, X_D01: x0 - x1 + K3P,
+            X_D10: x1 - x0 + K3P, X_S: x0 + x1, X_NS: 5 * P - x0 - x1, X_2S: 2 * (x0 + x1),
+            X_2N0: 2 * (K3P - x0), X_2N1: 2 * (K3P - x1)}[f]
+
+
+def form_bound(f):
+    B = SLOT_BOUND
+    return {X_0: B, X_1: B, X_2X0: 2 * B, X_2X1: 2 * B, X_N0: K3P + 1, X_N1: K3P + 1, X_D01: B + K3P,
+            X_D10: B + K3P, X_S: 2 * B, X_NS: 5 * P + 1, X_2S: 4 * B, X_2N0: 2 * K3P + 1, X_2N1: 2 * K3P + 1}[f]
+
+
+assert K3P >= SLOT_BOUND and 5 * P >= 2 * SLOT_BOUND
+assert all(form_bound(f) <= R for f in list(range(11)) + [12, 13])
+
+
+def gauss_products(x, y, xi, neg, dbl, conj):
+    """the three products of +-X Y, +-xi X Y or their conjugate, doubled with
+    dbl: (real part's, imaginary part's, shared) as (uform, uref, vform, vref)"""
+    if conj:                 # conj(X) conj(Y)
+        assert not (xi or neg or dbl)
+        return (X_1, x, X_D01, y), (X_0, x, X_NS, y), (X_D01, x, X_0, y)
+    if xi:                   # X Y with xi X = (x0 - x1, x0 + x1), the roles of X and Y exchanged
+        s2 = X_2S if dbl else X_S
+        if neg:
+            return ((X_2X0, x, X_2X1 if dbl else X_1, y), (X_2X1, x, X_2N0 if dbl else X_N0, y), (X_D10, x, s2, y))
+        return ((X_2X0, x, X_2N1 if dbl else X_N1, y), (X_2X1, x, X_2X0 if dbl else X_0, y), (X_D01, x, s2, y))
+    if neg:
+        return ((X_2X1 if dbl else X_1, x, X_S, y), (X_2X0 if dbl else X_0, x, X_D01, y),
+                (X_NS, x, X_2X0 if dbl else X_0, y))
+    return ((X_2N1 if dbl else X_N1, x, X_S, y), (X_2X0 if dbl else X_0, x, X_D10, y),
+            (X_S, x, X_2X0 if dbl else X_0, y))
+
+
+class Pair:
+    """an output in the paired-warp form: prods[h] of warp h = 0, 1 as (uform, uref,
+    vform, vref, store): store None, ("sum", slot) to store the accumulator once
+    this product is in, ("one", slot) to store this product alone; adds[h]: (slot,
+    sign) of the partner's partial sums; lins[h] (coefficient, ref), bias[h], and the
+    scale code (0: 1, 1: 3, 2: 6).  slot: the first free partial-sum slot."""
+
+    def __init__(self, o, slot=0):
+        self.dst, self.invfp, self.scale, self.slots = o.dst, o.mode == M_INVFP, 0, 0
+        self.own, self.both, self.anti = [[], []], [], []
+        self.prods, self.adds, self.lins, self.bias = [[], []], [[], []], [[], []], [0, 0]
+        cs = (o.c_re, o.c_im)
+        if self.invfp:
+            self.lins[0] = [(1, o.lins[0][1])]
+            return
+        if o.mode == M_LIN:
+            self.lins = [[(c * co, r) for co, r in o.lins] for c in cs]
+        else:
+            assert abs(cs[0]) == abs(cs[1]) and cs[0] > 0
+            self.scale = {1: 0, 3: 1, 6: 2}[cs[0]]
+            for t in o.terms:
+                self._term(t, cs[1] < 0)
+            for co, r in o.lins:
+                assert self.scale != 2 or co % 2 == 0
+                for h in range(2):
+                    self.lins[h].append((co // 2 if self.scale == 2 else co, r))
+        self._split(slot)
+        self._bounds()
+
+    def _term(self, t, conj):
+        neg = t.sign < 0
+        if t.kind == ONE:
+            assert not conj
+            self.lins[0].append((t.sign, t.x))
+            self.lins[1].append((t.sign, t.x))
+        elif t.kind == KARA:
+            re, im, s = gauss_products(t.x, t.y, t.xi, neg, t.dbl, conj)
+            self.own[0].append(re)
+            self.own[1].append(im)
+            self.both.append(s)
+        elif t.kind == SQR:
+            assert not conj
+            diff = (X_S, t.x, X_D10 if neg else X_D01, t.x)                     # +-(x0^2 - x1^2)
+            dbl = (X_N0, t.x, X_2X1, t.x) if neg else (X_2X0, t.x, X_1, t.x)    # +-2 x0 x1
+            if t.xi:
+                self.both.append(diff)
+                self.anti.append(dbl)
+            else:
+                self.own[0].append(diff)
+                self.own[1].append(dbl)
+        elif t.kind == FPMUL:
+            assert not t.xi and not neg
+            y = X_1 if t.yim else X_0
+            self.own[0].append((X_0, t.x, y, t.y))
+            self.own[1].append((X_N1 if conj else X_1, t.x, y, t.y))
+        else:               # NORM: x0^2 + x1^2 in the real part
+            assert t.kind == NORM and not neg and not conj
+            self.own[0] += [(X_0, t.x, X_0, t.x), (X_1, t.x, X_1, t.x)]
+
+    def _split(self, slot):
+        """the shared products dealt to the two warps so that the larger load is least"""
+        n, loads = len(self.both), [len(self.own[0]), len(self.own[1]) + len(self.anti)]
+        most = min(n, 1) if self.anti else n        # warp 1's share, after the subtracted sum: one product
+        s1 = min(range(most + 1), key=lambda k: (max(loads[0] + n - k, loads[1] + k), k))
+        share = [self.both[:n - s1], self.both[n - s1:]]
+
+        def put(h, prods, how, sign):
+            """prods of warp h, stored in the next slot for the other warp"""
+            for i, p in enumerate(prods):
+                last = i == len(prods) - 1
+                self.prods[h].append(p + ((how, slot + self.slots) if last else None,))
+            if prods:
+                self.adds[1 - h].append((slot + self.slots, sign))
+                self.slots += 1
+
+        put(0, share[0], "sum", 1)
+        put(1, self.anti, "sum", -1)
+        put(1, share[1], "one" if self.anti else "sum", 1)
+        for h in range(2):
+            self.prods[h] += [p + (None,) for p in self.own[h]]
+
+    def _bounds(self):
+        for h in range(2):
+            size = lambda ps: sum(form_bound(u) * form_bound(v) for u, _, v, _ in ps)       # noqa: E731
+            top, low = size(self.own[h] + self.both), 0
+            if h:
+                top += size(self.anti)
+            else:
+                low = size(self.anti)
+            assert top < ACC_LIMIT
+            hi = (top // R + P + 1) if top else 0
+            neg = -(-low // R)
+            if self.scale:
+                hi, neg = 3 * hi, 3 * neg
+            neg += sum(-co for co, _ in self.lins[h] if co < 0) * SLOT_BOUND
+            hi += sum(co for co, _ in self.lins[h] if co > 0) * SLOT_BOUND
+            self.bias[h] = -(-neg // P)
+            hi += self.bias[h] * P
+            assert hi * (2 if self.scale == 2 else 1) < POST_LIMIT
+            assert all(abs(co) <= 2 for co, _ in self.lins[h]) and len(self.lins[h]) < 4
+            assert len(self.prods[h]) < 16 and len(self.adds[h]) <= 2
+
+
+def pairs(outs):
+    """the outputs of a program in the paired-warp form, their partial-sum slots
+    numbered through"""
+    res, slot = [], 0
+    for o in outs:
+        res.append(None if o is None else Pair(o, slot))
+        slot += res[-1].slots if res[-1] else 0
+    return res
+
+
+class PairEmulator:
+    """Bit-exact model of the paired-warp form, with Emulator's interface."""
+
+    def __init__(self, progs):
+        self.progs = {name: pairs(outs) for name, outs, _ in progs}
+
+    def run(self, name, slots, bases):
+        at = lambda r: slots[bases[r >> 4] + (r & 15)]          # noqa: E731
+        res, part = {}, {}
+        for c in self.progs[name]:                              # the partial sums
+            for h in range(2 if c else 0):
+                acc = 0
+                for uf, ur, vf, vr, store in c.prods[h]:
+                    u, w = form_value(uf, at(ur)), form_value(vf, at(vr))
+                    assert 0 <= u < R and 0 <= w < R
+                    acc += u * w
+                    if store:
+                        assert store[1] not in part
+                        part[store[1]] = acc if store[0] == "sum" else u * w
+                part["acc", id(c), h] = acc
+        for c in self.progs[name]:
+            if c is None:
+                continue
+            v = [0, 0]
+            for h in range(2):
+                if c.invfp:
+                    v[h] = fp_inv_mont(at(c.lins[0][0][1])[0]) if h == 0 else 0
+                    continue
+                if c.prods[h]:
+                    acc = part["acc", id(c), h] + sum(sign * part[sl] for sl, sign in c.adds[h])
+                    m = (-acc * pow(P, -1, R)) % R
+                    assert (acc + m * P) % R == 0 and abs(acc) < ACC_LIMIT
+                    v[h] = ((acc + m * P) >> 384) * (1 if c.scale == 0 else 3)
+                v[h] += c.bias[h] * P + sum(co * at(r)[h] for co, r in c.lins[h])
+                v[h] = qp(v[h] * (2 if c.scale == 2 else 1))
+            res[bases[c.dst >> 4] + (c.dst & 15)] = tuple(v)
+        slots.update(res)                   # every warp computes before any writes
+
+
+def line_pair(k):
+    """Coefficient role k of the line-load op: pair k / 3, coefficient k % 3 of its
+    row.  c1 and c0 become l2 = c1 P.x and l3 = c0 P.y (one product a component by
+    the point's coordinate; LSCALE's value), c2 is stored as it is (None)."""
+    pair, c = divmod(k, 3)
+    if c == 2:
+        return None
+    d = Pair.__new__(Pair)
+    d.dst, d.invfp, d.scale, d.slots = ref(B_C, 6 * pair + (C_L3 if c == 0 else C_L2)), False, 0, 0
+    p = (X_LINE, 0, X_1 if c == 0 else X_0, ref(B_C, 6 * pair + C_PT), None)
+    d.prods, d.adds, d.lins, d.bias = [[p], [p]], [[], []], [[], []], [0, 0]
+    return d
+
+
+def encode_pair(c, h):
+    """the descriptor of warp h: header products | linear terms << 4 | scale << 6 | dst << 8 | bias << 16 |
+    inverse << 24; the two added slots, a byte each (15: none, and ends the list; 16 set: subtracted); then products combo (COMBOS) | vform << 4 | uref << 8 | vref << 16 | store << 24 (1: sum,
+    2: one) | slot << 26, with the uform's four bits in bits 15, 23, 30 and 31; then linear terms
+    coefficient & 15 | ref << 8"""
+    assert c.bias[h] < 256
+    w = [len(c.prods[h]) | (len(c.lins[h]) << 4) | (c.scale << 6) | (c.dst << 8) | (c.bias[h] << 16) |
+         (int(c.invfp) << 24)]
+    adds = [sl | (16 if sign < 0 else 0) for sl, sign in c.adds[h]] + [15, 15]
+    w.append(adds[0] | (adds[1] << 8) | (15 << 16))
+    for uf, ur, vf, vr, store in c.prods[h]:
+        combo = COMBO_LINE if uf == X_LINE else COMBOS.index((uf, vf)) if (uf, vf) in COMBOS else COMBO_GENERIC
+        assert combo not in (4,) or ur == vr        # (x0 + x1)(x0 - x1): one slot
+        x = combo | (vf << 4) | (ur << 8) | (vr << 16)
+        x |= ((uf & 1) << 15) | ((uf >> 1 & 1) << 23) | ((uf >> 2 & 1) << 30) | ((uf >> 3 & 1) << 31)
+        if store:
+            assert store[1] < PART_SLOTS
+            x |= ((1 if store[0] == "sum" else 2) << 24) | (store[1] << 26)
+        w.append(x)
+    return w + [(co & 15) | (r << 8) for co, r in c.lins[h]]
+
+
+# operand pairs with a case of their own in the kernel (kComboGeneric: by form)
+COMBOS = [(X_S, X_0), (X_N1, X_S), (X_0, X_D10), (X_2X0, X_1), (X_S, X_D01), (X_D01, X_S), (X_2X0, X_N1), (X_2X1, X_0),
+          (X_S, X_2X0), (X_2N1, X_S), (X_2X0, X_D10), (X_D01, X_2S), (X_2X0, X_2N1), (X_2X1, X_2X0)]
+COMBO_GENERIC, COMBO_LINE = 14, 15
+
+PART_SLOTS = 15     # partial-sum slots of an item (the square uses them all)
+
+
 # ---------------------------------------------------------------- constants
 def _f2_mul(a, b):
     return ((a[0] * b[0] - a[1] * b[1]) % P, (a[0] * b[1] + a[1] * b[0]) % P)
@@ -902,6 +1161,24 @@ def emit(path):
     for i in range(0, len(words), 6):
         L.append("    " + ", ".join("0x%08xu" % w for w in words[i:i + 6]) + ",")
     L.append("};")
+    words, index = [], []
+    for row in [pairs(outs) for _, outs, _ in progs] + [[line_pair(k) for k in range(6)]]:
+        index.append([])
+        for h in range(2):
+            for c in row:
+                index[-1].append(len(words) if c is not None else 0xffff)
+                words += encode_pair(c, h) if c is not None else []
+    L.append("// paired-warp form: per program, and last the line load, the first word of the descriptor of")
+    L.append("// coefficient k's warp h at 6 h + k (0xffff: no output)")
+    L.append("__device__ __constant__ uint16_t kPairIndex[%d][12] = {" % len(index))
+    for row in index:
+        L.append("    {%s}," % ", ".join("%d" % v for v in row))
+    L.append("};")
+    L.append("constexpr int kPartSlots = %d;" % PART_SLOTS)
+    L.append("__device__ __constant__ uint32_t kPair[%d] = {" % len(words))
+    for i in range(0, len(words), 6):
+        L.append("    " + ", ".join("0x%08xu" % w for w in words[i:i + 6]) + ",")
+    L.append("};")
     L.append("// accumulator coefficients per (kind, xi): alpha0..2, beta0..2, 4 bits each, in {-1, 0, 1}")
     L.append("__device__ __constant__ uint32_t kCoef[10] = {")
     row = []
@@ -925,8 +1202,6 @@ def emit(path):
     L.append("constexpr int kKSlotCount = %d;" % len(ks))
     L.append("// R^3 mod p: u * R^3 * R^-1 = u R^2 turns a plain inverse into Montgomery form")
     L.append("__device__ __constant__ uint32_t kR3[12] = {" + ", ".join(_limbs32(R * R * R % P)) + "};")
-    L.append("// 3p, the offset of SQR's x0 - x1 + 3p")
-    L.append("__device__ __constant__ uint32_t k3P[12] = {" + ", ".join(_limbs32(K3P)) + "};")
     L.append("// the verify op sequences (raw and normalised line tables): code | D << 5 | A << 8 | B << 11 |")
     L.append("// ci << 14; code < kNumPrograms is a program, kOpLoadLines loads line coefficient ci,")
     L.append("// kOpMillerDone marks the Miller value")
@@ -939,10 +1214,13 @@ def emit(path):
     L.append("constexpr uint32_t kNoWar = 0x%xu;" % NO_WAR)
     L.append("constexpr int kTGroup = %d;" % T_GROUP)
     max_bias = max(b for name, fn, _ in PROGRAMS for o in fn() if o is not None
-                   for b in (o.bias_re, o.bias_im, o.bias_lin_re, o.bias_lin_im))
+                   for b in [o.bias_re, o.bias_im, o.bias_lin_re, o.bias_lin_im] + Pair(o).bias)
     L.append("// largest bias multiple k of any output (the kernel keeps k p for k = 0 .. kMaxBias)")
     L.append("constexpr int kMaxBias = %d;" % max_bias)
     seqs = [driver_sequence(False), driver_sequence(True)]
+    for seq in seqs:   # verify_w.cu runs a line load and the LSCALE that follows it as one op
+        assert all((seq[i + 1][0] == [n for n, _, _ in PROGRAMS].index("LSCALE")) == (op[0] == OP_LOAD_LINES)
+                   for i, op in enumerate(seq[:-1]))
     for seq in seqs:   # verify_w.cu stores a program's outputs without a barrier after its reads
         assert all(no_war(op) for op in seq if (op[0] & ~COND_ML) < len(PROGRAMS))
     L.append("// Fp12 groups the sequences touch (operands, results, the inverse's temporaries)")

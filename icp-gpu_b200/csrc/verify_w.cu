@@ -1,24 +1,36 @@
-// Warp-uniform Fp2-lane verify kernel.  The same generated programs as
-// verify_fp2.cu (fp2ops.inc, gen_fp2ops.py), mapped the other way round: a
-// block of twelve warps verifies 32 items, warp w takes one role of the
-// twelve-thread decomposition (Fp2 coefficient k = w % 6 of every Fp12
-// result, half h = w / 6) and lane v works on item v.  Every lane of a warp
-// therefore runs the same output descriptor: descriptor reads are constant-
-// memory broadcasts, control flow never diverges, and the only per-lane
-// difference is which item's slots a lane reads and writes.
+// Warp-uniform Fp2-lane verify kernel.  The tower programs of gen_fp2ops.py in
+// their paired-warp form (fp2ops.inc): a block of twelve warps verifies 32 items,
+// one per lane.  The two warps of coefficient k (k = w % 6, w the warp) each
+// produce one component of the k-th Fp2 coefficient of every Fp12 result (half
+// h = w / 6: real, imaginary).  Every lane of a warp runs the same descriptor:
+// descriptor reads are constant-memory broadcasts, control flow never diverges,
+// and the only per-lane difference is which item's slots a lane reads and writes.
 //
 // Per verification (gpu-crypto/cuda/api.cu:80-91, api.cu:30-52, api.cu:65-78):
 // the Miller loop over both pairs with the lines of the generator's and the
 // key's tables, the reference's final-exponentiation chain, the canonical Gt
 // compared with one; optional Miller / Gt outputs.
 //
+// What bounds it: instruction throughput of three warps a scheduler.  Warps of
+// paired multiply-adds and warps of carry adds, run beside one another, slow each
+// other as if a paired multiply-add took 3.7 and an add 1.5 cycles of one shared
+// resource, and the kernel's time is its instructions at those rates (a product of
+// 108 pairs and about 150 adds: 657 cycles a warp and scheduler).  So every add
+// counts.  Against the form in which the two warps of a coefficient each added
+// every product into two accumulators (verify_fp2.cu's): one accumulator, no bias
+// to preload, one range reduction per component instead of two: 3.92 -> 3.60 ms
+// per 4,096 verifications.  Also measured, and slower: one warp a component with
+// no partial sums and a third more products, accumulated in place (4.34 ms);
+// eighteen warps, three to a coefficient, at the 96 registers that leaves (4.33 ms,
+// spills); operands of the next product loaded ahead (3.90 against 3.79 ms).
+//
 // Shared memory (16-byte units): the items' Fp2 slots interleaved by item
 // (unit ((s * 2 + c) * 3 + q) * 32 + v holds words 4q..4q+3 of component c of
 // slot s of item v, so a warp's load of one component is three conflict-free
-// 512-byte rows), then the block-shared constant slots, the partial-sum
-// exchange area (one 26-word partial per coefficient, half and item, same
-// interleaving), the per-item flags and the table of k p for the outputs'
-// bias multiples.
+// 512-byte rows), then the block-shared constant slots, the partial sums that
+// the warps of a coefficient hand each other (25 words, same interleaving), the
+// per-item flags and the tables of k p (the components' bias multiples) and of
+// the reduction.
 #include <cuda_runtime.h>
 
 #include "fp2ops.cuh"
@@ -37,7 +49,7 @@ constexpr int kCOff = 6 * kGroups;               // C area after the groups
 constexpr int kItemSlots = kCOff + 12;           // Fp2 slots per item
 constexpr int kSlotU4 = kItemSlots * 6 * kV;     // 16-byte units of the item slots
 constexpr int kKU4 = kKSlots * 6;                // constant slots, not interleaved
-constexpr int kXchU4 = 6 * 2 * 7 * kV;           // exchange: 26 words (7 units) per coefficient, half, item
+constexpr int kXchU4 = f2::kPartSlots * 7 * kV;  // partial sums: 25 words (7 units) per slot and item
 constexpr int kKpCount = f2::kMaxBias + 1;       // k p, 16 words each
 constexpr int kInfoWords = 4 * kV;               // per item: key index, flags, status, result flags
 constexpr int kFlagBytes = 16 * kV;              // per item and role: "not the expected value" bytes
@@ -51,7 +63,7 @@ static_assert(kSmemBytes <= 227 * 1024, "one block per SM");
 struct Sm {
     uint4* slots;      // item slots
     uint4* kslots;     // constant slots
-    uint4* xch;        // exchange
+    uint4* xch;        // partial sums
     uint4* qp;         // QP table (qp_reduce_tab)
     uint32_t* kp;      // k p table
     uint32_t* info;    // per item: [0] key index, [1] skip bits, [2] status, [3] spare
@@ -103,202 +115,239 @@ __device__ __forceinline__ void load_kp(uint32_t* t, const Sm& s, uint32_t k) {
 
 __device__ __forceinline__ int sext4(uint32_t v) { return (int)(v << 28) >> 28; }
 
-// P into the two accumulators with coefficients ca, cb (bit 0 nonzero, bit 1 negative)
-__device__ __forceinline__ void acc_pair(uint32_t* acc0, uint32_t* acc1, const uint32_t* P, uint32_t ca,
-                                         uint32_t cb) {
-    if (ca & 1u) {
-        if (ca >> 1) f2::acc_sub(acc0, P);
-        else f2::acc_plus(acc0, P);
+// An operand: the linear form `f` of a slot's two components (gen_fp2ops.py)
+__device__ __forceinline__ void load_form(uint32_t* x, const Sm& s, uint32_t f, uint32_t slot) {
+    const int c = f & 1u;
+    if (f >= 8u && f < 12u) {                       // x0 + x1, 5p - x0 - x1, 2 (x0 + x1)
+        uint32_t y[12];
+        load_fp(x, s, slot, 0);
+        load_fp(y, s, slot, 1);
+        f2::add12(x, x, y);
+        if (f == 9u) f2::sub_from_5p(x);
+        if (f == 10u) f2::dbl12(x);
+        return;
     }
-    if (cb & 1u) {
-        if (cb >> 1) f2::acc_sub(acc1, P);
-        else f2::acc_plus(acc1, P);
+    load_fp(x, s, slot, c);
+    if (f < 2u) return;                             // x_c
+    if (f >= 6u && f < 8u) {                        // x_c - x_(1-c) + 3p
+        uint32_t y[12];
+        load_fp(y, s, slot, 1 - c);
+        f2::add3p_sub(x, x, y);
+        return;
+    }
+    if (f >= 4u) f2::sub_from_3p(x);          // 3p - x_c
+    if ((f & 4u) == 0u || f >= 12u) f2::dbl12(x);   // 2 x_c, 2 (3p - x_c)
+}
+
+// The operands U, V of the product described by w (gen_fp2ops.py: COMBOS).  The
+// pairs of forms that the hot programs use have a case each, with all loads
+// ahead of the arithmetic (two calls of load_form cost a lone warp 580 cycles a
+// product, these cases 380; 3.65 -> 3.60 ms).
+__device__ __forceinline__ void load_operands(uint32_t* U, uint32_t* V, const Sm& s, uint32_t w, const Bases& bs,
+                                              const uint32_t* line) {
+    const uint32_t xs = slot_addr(bs, (w >> 8) & 0x7fu), ys = slot_addr(bs, (w >> 16) & 0x7fu);
+    uint32_t T[12];
+    switch (w & 15u) {
+        case 0:     // x0 + x1, y0
+            load_fp(U, s, xs, 0); load_fp(T, s, xs, 1); load_fp(V, s, ys, 0);
+            f2::add12(U, U, T);
+            break;
+        case 1:     // 3p - x1, y0 + y1
+            load_fp(U, s, xs, 1); load_fp(V, s, ys, 0); load_fp(T, s, ys, 1);
+            f2::sub_from_3p(U);
+            f2::add12(V, V, T);
+            break;
+        case 2:     // x0, y1 - y0 + 3p
+            load_fp(U, s, xs, 0); load_fp(T, s, ys, 0); load_fp(V, s, ys, 1);
+            f2::add3p_sub(V, V, T);
+            break;
+        case 3:     // 2 x0, y1
+            load_fp(U, s, xs, 0); load_fp(V, s, ys, 1);
+            f2::dbl12(U);
+            break;
+        case 4:     // x0 + x1, x0 - x1 + 3p
+            load_fp(V, s, xs, 0); load_fp(T, s, xs, 1);
+            f2::add12(U, V, T);
+            f2::add3p_sub(V, V, T);
+            break;
+        case 5: {   // x0 - x1 + 3p, y0 + y1
+            uint32_t S[12];
+            load_fp(U, s, xs, 0); load_fp(T, s, xs, 1); load_fp(V, s, ys, 0); load_fp(S, s, ys, 1);
+            f2::add3p_sub(U, U, T);
+            f2::add12(V, V, S);
+            break;
+        }
+        case 6:     // 2 x0, 3p - y1
+            load_fp(U, s, xs, 0); load_fp(V, s, ys, 1);
+            f2::dbl12(U);
+            f2::sub_from_3p(V);
+            break;
+        case 7:     // 2 x1, y0
+            load_fp(U, s, xs, 1); load_fp(V, s, ys, 0);
+            f2::dbl12(U);
+            break;
+        case 8:     // x0 + x1, 2 y0
+            load_fp(U, s, xs, 0); load_fp(T, s, xs, 1); load_fp(V, s, ys, 0);
+            f2::add12(U, U, T);
+            f2::dbl12(V);
+            break;
+        case 9:     // 2 (3p - x1), y0 + y1
+            load_fp(U, s, xs, 1); load_fp(V, s, ys, 0); load_fp(T, s, ys, 1);
+            f2::sub_from_3p(U);
+            f2::dbl12(U);
+            f2::add12(V, V, T);
+            break;
+        case 10:    // 2 x0, y1 - y0 + 3p
+            load_fp(U, s, xs, 0); load_fp(T, s, ys, 0); load_fp(V, s, ys, 1);
+            f2::dbl12(U);
+            f2::add3p_sub(V, V, T);
+            break;
+        case 11: {  // x0 - x1 + 3p, 2 (y0 + y1)
+            uint32_t S[12];
+            load_fp(U, s, xs, 0); load_fp(T, s, xs, 1); load_fp(V, s, ys, 0); load_fp(S, s, ys, 1);
+            f2::add3p_sub(U, U, T);
+            f2::add12(V, V, S);
+            f2::dbl12(V);
+            break;
+        }
+        case 12:    // 2 x0, 2 (3p - y1)
+            load_fp(U, s, xs, 0); load_fp(V, s, ys, 1);
+            f2::dbl12(U);
+            f2::sub_from_3p(V);
+            f2::dbl12(V);
+            break;
+        case 13:    // 2 x1, 2 y0
+            load_fp(U, s, xs, 1); load_fp(V, s, ys, 0);
+            f2::dbl12(U);
+            f2::dbl12(V);
+            break;
+        case 14:
+            load_form(U, s, ((w >> 15) & 1u) | ((w >> 22) & 2u) | ((w >> 28) & 12u), xs);
+            load_form(V, s, (w >> 4) & 15u, ys);
+            break;
+        default:    // the line coefficient, the point's coordinate
+#pragma unroll
+            for (int i = 0; i < 12; ++i) U[i] = line[i];
+            load_fp(V, s, ys, (w >> 4) & 1u);
     }
 }
 
-// partial sum `acc` (26 words) of this lane into exchange unit row `row`
-__device__ __forceinline__ void xch_store(uint4* row, const uint32_t* acc) {
+// a partial sum (25 words) of this lane into its slot, and back
+__device__ __forceinline__ uint4* part_row(const Sm& s, uint32_t slot) { return s.xch + slot * 7 * kV + s.v; }
+__device__ __forceinline__ void part_store(uint4* row, const uint32_t* p, uint32_t top) {
 #pragma unroll
-    for (int q = 0; q < 6; ++q) row[q * kV] = make_uint4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
-    row[6 * kV] = make_uint4(acc[24], acc[25], 0u, 0u);
+    for (int q = 0; q < 6; ++q) row[q * kV] = make_uint4(p[4 * q], p[4 * q + 1], p[4 * q + 2], p[4 * q + 3]);
+    reinterpret_cast<uint32_t*>(row + 6 * kV)[0] = top;
 }
-__device__ __forceinline__ void xch_load(uint32_t* p, const uint4* row) {
+__device__ __forceinline__ void part_load(uint32_t* p, const uint4* row) {
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
         const uint4 u = row[q * kV];
         p[4 * q] = u.x; p[4 * q + 1] = u.y; p[4 * q + 2] = u.z; p[4 * q + 3] = u.w;
     }
-    const uint4 u = row[6 * kV];
-    p[24] = u.x;
-    p[25] = u.y;
+    p[24] = reinterpret_cast<const uint32_t*>(row + 6 * kV)[0];
 }
 
-// Phase 1 of an output (product modes): this half's products into both
-// accumulators; the partner's component (accX) goes to the exchange row.
-__device__ __forceinline__ void accumulate(uint32_t off, const Sm& s, const Bases& bs, uint4* xch_out, int half,
-                                           uint32_t* own) {
-    const uint32_t hdr = f2::kDesc[off], bias = f2::kDesc[off + 1];
-    const uint32_t nt = (hdr >> 2) & 15u;
-    uint32_t accO[26], accX[26];
-    const uint32_t sw = half ? 8u : 0u, c0 = half ? 12u : 0u, c1 = half ? 0u : 12u;
-#pragma unroll
-    for (int i = 0; i < 12; ++i) accO[i] = accX[i] = 0;
-    accO[25] = accX[25] = 0;
-    load_kp(accO + 12, s, (bias >> sw) & 0xffu);
-    load_kp(accX + 12, s, (bias >> (8u - sw)) & 0xffu);
-    for (uint32_t t = 0; t < nt; ++t) {
-        const uint32_t w = f2::kDesc[off + 2 + t];
-        const uint32_t kind = w & 7u, xi = (w >> 3) & 1u, neg = (w >> 4) & 1u, dbl = (w >> 5) & 1u,
-                       yim = (w >> 6) & 1u, mask = (w >> 24) & 7u;
-        const uint32_t xs = slot_addr(bs, (w >> 8) & 0x7fu), ys = slot_addr(bs, (w >> 16) & 0x7fu);
-        if (kind == f2::kOne) {             // X R: X into the high half of both accumulators
-            uint32_t x0[12], x1[12];
-            load_fp(x0, s, xs, half);
-            load_fp(x1, s, xs, 1 - half);
-            f2::acc_add_hi(accO, x0, neg);
-            f2::acc_add_hi(accX, x1, neg);
-            continue;
-        }
-        const uint32_t cw = f2::kCoef[2 * kind + xi] ^ (neg ? 0x666666u : 0u);
-        const uint32_t np = kind == f2::kKara ? 3u : 2u;
+// acc (25 words) = the sum of the np > 0 products described at `prod`, partial
+// sums stored on the way.  line: the key-table coefficient this warp has read,
+// for the line load's products.
+__device__ __forceinline__ void sum_products(uint32_t* acc, const uint32_t* prod, uint32_t np, const Sm& s,
+                                             const Bases& bs, const uint32_t* line) {
 #pragma unroll 1
-        for (uint32_t j = 0; j < np; ++j) {
-            if (!((mask >> j) & 1u)) continue;
-            uint32_t U[12], V[12], P[24];
-            if (kind == f2::kSqr) {          // U = x0 + x1, 2 x0
-                load_fp(U, s, xs, 0);
-                if (j == 0) {
-                    uint32_t T[12];
-                    load_fp(T, s, xs, 1);
-                    f2::add12(U, U, T);
-                } else {
-                    f2::dbl12(U);
-                }
-            } else if (kind == f2::kKara && xi) {   // xi X = (x0 - x1 + 3p, x0 + x1); sum 2 x0 + 3p
-                load_fp(U, s, xs, 0);
-                if (j == 2) {
-                    const uint32_t z[12] = {0};
-                    f2::dbl12(U);
-                    f2::add3p_sub(U, U, z);
-                } else {
-                    uint32_t T[12];
-                    load_fp(T, s, xs, 1);
-                    if (j == 0) f2::add3p_sub(U, U, T);
-                    else f2::add12(U, U, T);
-                }
-            } else {                         // x0, x1 (KARA: sum x0 + x1)
-                load_fp(U, s, xs, j & 1u);
-                if (j == 2) {
-                    uint32_t T[12];
-                    load_fp(T, s, xs, 1);
-                    f2::add12(U, U, T);
-                }
-            }
-            if (kind == f2::kKara) {        // V = y0, y1, y0 + y1 (doubled when dbl)
-                load_fp(V, s, ys, j & 1u);
-                if (j == 2) {
-                    uint32_t T[12];
-                    load_fp(T, s, ys, 1);
-                    f2::add12(V, V, T);
-                }
-                if (dbl) f2::dbl12(V);
-            } else if (kind == f2::kSqr) {  // V = x0 - x1 + 3p, x1
-                load_fp(V, s, xs, 1);
-                if (j == 0) {
-                    uint32_t T[12];
-                    load_fp(T, s, xs, 0);
-                    f2::add3p_sub(V, T, V);
-                }
-            } else if (kind == f2::kFpMul) {
-                load_fp(V, s, ys, yim);
-            } else {                        // NORM: x_j^2
-                load_fp(V, s, xs, j);
-            }
-            f2::prod24k(P, U, V);
-            acc_pair(accO, accX, P, (cw >> (c0 + 4 * j)) & 3u, (cw >> (c1 + 4 * j)) & 3u);
-        }
-    }
-    xch_store(xch_out, accX);
+    for (uint32_t j = 0; j < np; ++j) {
+        const uint32_t w = prod[j];
+        uint32_t U[12], V[12], P[24];
+        load_operands(U, V, s, w, bs, line);
+        f2::prod24k(P, U, V);
+        if (j == 0) {
 #pragma unroll
-    for (int i = 0; i < 26; ++i) own[i] = accO[i];
+            for (int i = 0; i < 24; ++i) acc[i] = P[i];
+            acc[24] = 0;
+        } else {
+            f2::add25(acc, P);
+        }
+        const uint32_t store = (w >> 24) & 3u;
+        if (store == 1u) part_store(part_row(s, (w >> 26) & 15u), acc, acc[24]);
+        if (store == 2u) part_store(part_row(s, (w >> 26) & 15u), P, 0u);
+    }
 }
 
-// Phase 2: component `half` of the output into o (12 words).  own: this
-// half's accumulator of that component (product modes), xch_in: the partner's.
-__device__ __forceinline__ void finish(uint32_t off, const Sm& s, const Bases& bs, int half, uint32_t* own,
-                                       const uint4* xch_in, uint32_t* o) {
-    const uint32_t hdr = f2::kDesc[off], bias = f2::kDesc[off + 1];
-    const uint32_t mode = hdr & 3u, nt = (hdr >> 2) & 15u, nl = (hdr >> 6) & 3u;
-    const int cc = half ? sext4(hdr >> 20) : sext4(hdr >> 16);
-    const uint32_t bias_lin = (bias >> (16 + 8 * half)) & 0xffu;
-    const uint32_t* lin = f2::kDesc + off + 2 + nt;
-
-    if (mode == f2::kModeInvFp) {
-        if (half == 0) {
-            fp z;
-            load_fp(z.w, s, slot_addr(bs, lin[0] >> 8), 0);
-            fp r = fp_inverse_warp(z, f2::kR3);
+// Warp (k, half) on program `pid` for every item of the block.  No program of
+// the generated sequences writes a slot that any warp of it reads (the
+// generator places a result that would overwrite an operand in an unused group,
+// and refuses to emit a sequence where it cannot), so a warp stores its
+// component as soon as it has it: one block-wide meeting per program, after the
+// stores, and one of a coefficient's two warps when the partial sums are there.
+__device__ __forceinline__ void run(int pid, const Sm& s, int k, int half, const Bases& bs, const uint32_t* line) {
+    const uint32_t off = f2::kPairIndex[pid][6 * half + k];
+    const uint32_t hdr = off != 0xffffu ? f2::kPair[off] : 0u, adds = off != 0xffffu ? f2::kPair[off + 1] : 0u;
+    const uint32_t np = hdr & 15u;
+    uint32_t acc[25];
+    if (np) sum_products(acc, f2::kPair + off + 2, np, s, bs, line);
+    // a named barrier (id 1 + k) over the 64 threads of coefficient k; both
+    // warps reach it on every program, whether or not they have an output
+    asm volatile("bar.sync %0, 64;" ::"r"(1 + k) : "memory");
+    if (off != 0xffffu) {
+        const uint32_t nl = (hdr >> 4) & 3u, scale = (hdr >> 6) & 3u, bias = (hdr >> 16) & 0xffu;
+        const uint32_t* lin = f2::kPair + off + 2 + np;
+        uint32_t o[12];
+        if ((hdr >> 24) & 1u) {                     // the one Fp inverse, all 32 items together
+            fp r = fp_zero();
+            if (half == 0) {
+                fp z;
+                load_fp(z.w, s, slot_addr(bs, lin[0] >> 8), 0);
+                r = fp_inverse_warp(z, f2::kR3);
+            }
 #pragma unroll
             for (int i = 0; i < 12; ++i) o[i] = r.w[i];
         } else {
+            uint32_t r[13];
+            if (np) {
+#pragma unroll 1
+                for (int i = 0; i < 2; ++i) {
+                    const uint32_t a = (adds >> (8 * i)) & 31u;
+                    if (a == 15u) break;
+                    uint32_t p[25];
+                    part_load(p, part_row(s, a & 15u));
+                    if (a & 16u) f2::sub25_25(acc, p);
+                    else f2::add25_25(acc, p);
+                }
+                f2::redc26(r, acc);
+                if (scale) {                        // 3 r
+                    uint32_t d[13];
 #pragma unroll
-            for (int i = 0; i < 12; ++i) o[i] = 0;
+                    for (int i = 0; i < 13; ++i) d[i] = r[i];
+                    f2::dbl13(d);
+                    f2::add13(r, d);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 13; ++i) r[i] = 0;
+            }
+            if (bias) {
+                uint32_t b[13];
+                load_kp(b, s, bias);
+                f2::add13(r, b);
+            }
+#pragma unroll 1
+            for (uint32_t j = 0; j < nl; ++j) {
+                uint32_t z[12];
+                load_fp(z, s, slot_addr(bs, lin[j] >> 8), half);
+                const int c = sext4(lin[j]);
+                if (c & 1) {
+                    if (c < 0) f2::sub13_12(r, z);
+                    else f2::add13_12(r, z);
+                } else {
+                    f2::dbl12(z);
+                    if (c < 0) f2::sub13_12(r, z);
+                    else f2::add13_12(r, z);
+                }
+            }
+            if (scale == 2u) f2::dbl13(r);          // 2 (3 REDC + ..)
+            f2::qp_reduce_tab(o, r, s.qp);
         }
-        return;
+        store_fp(s, slot_addr(bs, (hdr >> 8) & 0x7fu), half, o);
     }
-    uint32_t r[13];
-    if (mode == f2::kModeLin) {
-        load_kp(r, s, bias_lin);
-        for (uint32_t j = 0; j < nl; ++j) {
-            uint32_t z[12];
-            load_fp(z, s, slot_addr(bs, lin[j] >> 8), half);
-            f2::madd13(r, z, cc * sext4(lin[j]));
-        }
-    } else {
-        uint32_t p[26];
-        xch_load(p, xch_in);
-        f2::add26(own, p);
-        uint32_t red[13];
-        f2::redc26(red, own);
-        if (mode == f2::kModeSimple) {
-            f2::qp_reduce_tab(o, red, s.qp);
-            return;
-        }
-        uint32_t q[12];
-        f2::qp_reduce_tab(q, red, s.qp);
-        load_kp(r, s, bias_lin);
-        f2::madd13(r, q, cc);
-        for (uint32_t j = 0; j < nl; ++j) {
-            uint32_t z[12];
-            load_fp(z, s, slot_addr(bs, lin[j] >> 8), half);
-            f2::madd13(r, z, sext4(lin[j]));
-        }
-    }
-    f2::qp_reduce_tab(o, r, s.qp);
-}
-
-// program `pid` for every item of the block: accumulate, exchange (the two
-// warps of coefficient k meet), reduce, meet, write, meet.  The descriptor
-// index of the role is 8 half + k.  No program of the generated sequences
-// writes a slot that any role of it reads (the generator places a result
-// that would overwrite an operand in an unused group, and refuses to emit a
-// sequence where it cannot), so a role stores its output as soon as it has
-// it: one block-wide meeting per program, after the stores.
-__device__ __forceinline__ void run(int pid, const Sm& s, int k, int half, const Bases& bs) {
-    const uint32_t off = f2::kOutIndex[pid][8 * half + k];
-    const uint32_t mode = off != 0xffffu ? (f2::kDesc[off] & 3u) : 0u;
-    const bool prod = off != 0xffffu && (mode == f2::kModeSimple || mode == f2::kModeFull);
-    uint4* mine = s.xch + (k * 2 + half) * 7 * kV + s.v;
-    const uint4* theirs = s.xch + (k * 2 + (1 - half)) * 7 * kV + s.v;
-    uint32_t own[26];
-    if (prod) accumulate(off, s, bs, mine, half, own);
-    // only warps k and 6 + k exchange partial sums here: a named barrier
-    // (id 1 + k) over those 64 threads instead of the whole block; both warps
-    // reach it on every program, whether or not their role has an output
-    asm volatile("bar.sync %0, 64;" ::"r"(1 + k) : "memory");
-    uint32_t o[12];
-    if (off != 0xffffu) finish(off, s, bs, half, own, theirs, o);
-    if (off != 0xffffu) store_fp(s, slot_addr(bs, (f2::kDesc[off] >> 8) & 0x7fu), half, o);
     __syncthreads();
 }
 
@@ -409,7 +458,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_verify_w(VerifyArgs a, const ui
     s.info = s.kp + 16 * kKpCount;
     s.flags = reinterpret_cast<uint8_t*>(s.info + kInfoWords);
     s.bcast = reinterpret_cast<uint32_t*>(s.flags + kFlagBytes);
-    const int role = threadIdx.x >> 5;
+    // from a shuffle, so that the compiler knows it to be uniform in the warp:
+    // descriptor decoding and branches on uniform registers (3.75 -> 3.65 ms)
+    const int role = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
     const int half = role / 6, k = role % 6;
     s.v = threadIdx.x & 31;
 
@@ -517,42 +568,36 @@ __global__ void __launch_bounds__(kThreads, 1) k_verify_w(VerifyArgs a, const ui
             const uint32_t e = f2::kSeq[norm][st];
             const uint32_t code = e & 31u;
             if ((e & f2::kCondMl) && !a.ml_out) continue;
+            Bases bs;
+            bs.b = (uint64_t)grp((e >> 5) & 7u) | (uint64_t)grp((e >> 8) & 7u) << 8 |
+                   (uint64_t)grp((e >> 11) & 7u) << 16 | (uint64_t)(kKSlots + kCOff) << 24 |
+                   (uint64_t)grp(f2::kTGroup) << 40;
+            int pid = (int)code;
+            uint32_t line[12];
             if (code == f2::kOpLoadLines) {
                 // role (k, h): pair k / 3, coefficient k % 3, component h; a
                 // skipped pair gets the line (0, 0, 1), which leaves f unchanged.
-                // When the next op is LSCALE (l2 = c1 P.x, l3 = c0 P.y), the roles
-                // holding c1 and c0 form their component of it here: that
-                // program's every output is one product with a zero bias, so
-                // QP(REDC(c_h * P coordinate)) is bit for bit its result, and the
-                // program's exchange and barriers are saved.
-                const bool fuse = st + 1 < seq_len && (f2::kSeq[norm][st + 1] & 31u) == (uint32_t)f2::P_LSCALE;
+                // The roles holding c1 and c0 form their component of l2 = c1 P.x
+                // and l3 = c0 P.y (the LSCALE op that follows, and is skipped).
                 const int pair = k / 3, c = k % 3;
-                const uint32_t C = kKSlots + kCOff + 6 * pair;
-                uint32_t x[12];
                 if ((skip >> pair) & 1u) {
                     const fp v = (c == 2 && half == 0) ? fp_one() : fp_zero();
 #pragma unroll
-                    for (int i = 0; i < 12; ++i) x[i] = v.w[i];
+                    for (int i = 0; i < 12; ++i) line[i] = v.w[i];
                 } else {
                     const uint64_t* q = pair ? pk : g2_lines;
                     const uint4* g = reinterpret_cast<const uint4*>(q + 36 * ((e >> 14) & 127u) + 12 * c + 6 * half);
                     const uint4 a0 = __ldg(g), a1 = __ldg(g + 1), a2 = __ldg(g + 2);
-                    x[0] = a0.x; x[1] = a0.y; x[2] = a0.z; x[3] = a0.w;
-                    x[4] = a1.x; x[5] = a1.y; x[6] = a1.z; x[7] = a1.w;
-                    x[8] = a2.x; x[9] = a2.y; x[10] = a2.z; x[11] = a2.w;
+                    line[0] = a0.x; line[1] = a0.y; line[2] = a0.z; line[3] = a0.w;
+                    line[4] = a1.x; line[5] = a1.y; line[6] = a1.z; line[7] = a1.w;
+                    line[8] = a2.x; line[9] = a2.y; line[10] = a2.z; line[11] = a2.w;
                 }
-                store_fp(s, C + c, half, x);
-                if (fuse && c < 2) {
-                    uint32_t y[12], P[26], red[13], o[12];
-                    load_fp(y, s, C + 3, c == 1 ? 0 : 1);   // P.x for l2, P.y for l3
-                    f2::prod24k(P, x, y);
-                    P[24] = P[25] = 0;
-                    f2::redc26(red, P);
-                    f2::qp_reduce_tab(o, red, s.qp);
-                    store_fp(s, C + (c == 1 ? 4 : 5), half, o);
-                }
-                __syncthreads();
-                if (fuse) ++st;
+                if (c == 2) store_fp(s, kKSlots + kCOff + 6 * pair + 2, half, line);
+                pid = f2::kNumPrograms;             // the line load's row of the descriptor index
+                ++st;
+            }
+            if (code < (uint32_t)f2::kNumPrograms || code == f2::kOpLoadLines) {
+                run(pid, s, k, half, bs, line);
             } else if (code == f2::kOpLoadCorr) {
                 // the generator's and the key's Miller correction factors into the c2 slots
                 if (k < 2) {
@@ -563,12 +608,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_verify_w(VerifyArgs a, const ui
                 __syncthreads();
             } else if (code == f2::kOpMillerDone) {
                 if (a.ml_out) emit_group(s, (e >> 5) & 7u, k, half, have ? a.ml_out + 72 * (size_t)item : nullptr);
-            } else {
-                Bases bs;
-                bs.b = (uint64_t)grp((e >> 5) & 7u) | (uint64_t)grp((e >> 8) & 7u) << 8 |
-                       (uint64_t)grp((e >> 11) & 7u) << 16 | (uint64_t)(kKSlots + kCOff) << 24 |
-                       (uint64_t)grp(f2::kTGroup) << 40;
-                run((int)code, s, k, half, bs);
             }
         }
         const bool one = emit_group(s, (int)f2::kGtGroup[norm], k, half,
