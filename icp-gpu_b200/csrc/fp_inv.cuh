@@ -1,189 +1,156 @@
-// Fp inverse by the binary extended Euclidean algorithm, shared by the verify
-// kernels (the final exponentiation's one inversion) and the hash to G1 (the
-// affine result): a few hundred shift-and-subtract passes on 12-limb values
-// instead of the ~570 Montgomery multiplications of a Fermat power; and its
-// warp-wide form, the inverses of a whole warp's values for one Euclid.  The
-// caller passes R^3 mod p (12 limbs, from its generated constants).
+// Fp inverse by Bernstein and Yang's division steps ("Fast constant-time gcd
+// computation and modular inversion", CHES 2019), shared by the verify kernels
+// (the final exponentiation's one inversion), the line tables and the hash to G1.
+//
+// One step takes (delta, f, g), f odd, to
+//   (2 - delta, g, (g - f) / 2)             when delta > 0 and g is odd,
+//   (2 + delta, f, (g + (g mod 2) f) / 2)   otherwise
+// (delta counted in halves, from 1), and after enough steps g = 0 and f = +-gcd.
+// Thirty steps look at no more than the low thirty bits of f and g, so they run on
+// one word each and leave a 2 x 2 matrix of words, which is then applied to the
+// whole of f and g (an exact division by 2^30) and, with a multiple of p added to
+// make the division exact, to d and e, where f = d x and g = e x modulo p.
+//
+// Values are signed, in thirteen limbs of thirty bits, so that a limb product is
+// one signed wide multiply-add and there are no carry chains.  Nothing branches
+// on the value but the end of the loop (26 or 27 rounds for 381 bits), so the
+// lanes of a warp invert different values side by side: 67 k cycles (34 us) a
+// warp, bound by one warp's dependent chain.  A binary Euclid diverges; on the
+// product of the warp's values (prefix and suffix products by shuffles), which
+// avoids that, it took 287 k cycles, and the verify kernel 3.60 instead of 3.50 ms.
 #pragma once
 #include "fp.cuh"
 
 namespace bls {
 
-// ---------------------------------------------------------------------------
-// Fp inverse by the binary extended Euclidean algorithm (Knuth, TAOCP vol. 2,
-// 4.5.2; Menezes et al., Handbook of Applied Cryptography, Alg. 14.61 in its
-// modular form).  Variable time: the inputs are public.  x: Montgomery form
-// of a (any value below 2^381 + p); returns a^-1 in Montgomery form (0 for 0).
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ bool u_is_one(const uint32_t* u) {
-    uint32_t o = u[0] ^ 1u;
+constexpr int kInvLimbs = 13, kInvBits = 30;
+constexpr int32_t kInvMask = (1 << kInvBits) - 1;
+// (49 * 381 + 57) / 17 = 1,101 steps suffice from delta = 1, fewer from 1/2
+// (Theorem 11.2 there); the loop ends when g is zero
+constexpr int kInvMaxRounds = 37;
+
+__device__ __forceinline__ void inv_limbs(int32_t* r, const uint32_t* w) {
 #pragma unroll
-    for (int i = 1; i < 12; ++i) o |= u[i];
-    return o == 0;
-}
-__device__ __forceinline__ bool geq12(const uint32_t* a, const uint32_t* b) {
-    uint32_t br = 0;
-#pragma unroll
-    for (int i = 0; i < 12; ++i) br = (uint32_t)(((uint64_t)a[i] - b[i] - br) >> 63);
-    return br == 0;
-}
-__device__ __forceinline__ void sub12(uint32_t* a, const uint32_t* b) {
-    uint32_t br = 0;
-#pragma unroll
-    for (int i = 0; i < 12; ++i) {
-        uint64_t t = (uint64_t)a[i] - b[i] - br;
-        a[i] = (uint32_t)t;
-        br = (uint32_t)(t >> 63);
-    }
-}
-// x = x / 2 mod p for x < p
-__device__ __forceinline__ void half_mod(uint32_t* x) {
-    const uint32_t P_[12] = {BLS_P0, BLS_P1, BLS_P2, BLS_P3, BLS_P4, BLS_P5,
-                             BLS_P6, BLS_P7, BLS_P8, BLS_P9, BLS_P10, BLS_P11};
-    const uint32_t odd = 0u - (x[0] & 1u);
-    uint32_t c = 0;
-#pragma unroll
-    for (int i = 0; i < 12; ++i) {
-        uint64_t t = (uint64_t)x[i] + (P_[i] & odd) + c;
-        x[i] = (uint32_t)t;
-        c = (uint32_t)(t >> 32);
-    }
-#pragma unroll
-    for (int i = 0; i < 11; ++i) x[i] = __funnelshift_r(x[i], x[i + 1], 1);
-    x[11] = (x[11] >> 1) | (c << 31);
-}
-__device__ __forceinline__ void shr1(uint32_t* u) {
-#pragma unroll
-    for (int i = 0; i < 11; ++i) u[i] = __funnelshift_r(u[i], u[i + 1], 1);
-    u[11] >>= 1;
-}
-// x1 = x1 - x2 mod p (both < p)
-__device__ __forceinline__ void sub_mod(uint32_t* x1, const uint32_t* x2) {
-    const uint32_t P_[12] = {BLS_P0, BLS_P1, BLS_P2, BLS_P3, BLS_P4, BLS_P5,
-                             BLS_P6, BLS_P7, BLS_P8, BLS_P9, BLS_P10, BLS_P11};
-    uint32_t br = 0;
-#pragma unroll
-    for (int i = 0; i < 12; ++i) {
-        uint64_t t = (uint64_t)x1[i] - x2[i] - br;
-        x1[i] = (uint32_t)t;
-        br = (uint32_t)(t >> 63);
-    }
-    const uint32_t m = 0u - br;
-    uint32_t c = 0;
-#pragma unroll
-    for (int i = 0; i < 12; ++i) {
-        uint64_t t = (uint64_t)x1[i] + (P_[i] & m) + c;
-        x1[i] = (uint32_t)t;
-        c = (uint32_t)(t >> 32);
+    for (int i = 0; i < kInvLimbs; ++i) {
+        const int b = kInvBits * i, k = b >> 5, s = b & 31;
+        const uint32_t lo = w[k], hi = k + 1 < 12 ? w[k + 1] : 0u;
+        r[i] = (int32_t)(__funnelshift_r(lo, hi, s) & (uint32_t)kInvMask);
     }
 }
 
+// x: Montgomery form of a (any value below 2^381 + p); a^-1 in Montgomery form,
+// 0 for 0.  kR3: R^3 mod p, which takes the plain inverse x^-1 there.
 static __device__ __noinline__ fp fp_inverse_mont(fp x, const uint32_t* kR3) {
     // canonical representative (x < 2^381 + p < 3p)
-    uint32_t d[12];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        uint32_t br = sub_p(d, x.w);
-#pragma unroll
-        for (int i = 0; i < 12; ++i) x.w[i] = br ? x.w[i] : d[i];
-    }
-    if (fp_is_zero(x)) return x;
-    uint32_t u[12], v[12], x1[12], x2[12];
+    reduce_once(x.w);
+    reduce_once(x.w);
+    uint32_t t[13];
     const uint32_t P_[12] = {BLS_P0, BLS_P1, BLS_P2, BLS_P3, BLS_P4, BLS_P5,
                              BLS_P6, BLS_P7, BLS_P8, BLS_P9, BLS_P10, BLS_P11};
+    int32_t P30[kInvLimbs], f[kInvLimbs], g[kInvLimbs], d[kInvLimbs], e[kInvLimbs];
+    inv_limbs(P30, P_);
+    inv_limbs(g, x.w);
+#pragma unroll
+    for (int i = 0; i < kInvLimbs; ++i) {
+        f[i] = P30[i];
+        d[i] = 0;
+        e[i] = i == 0 ? 1 : 0;
+    }
+    int delta = 1;
+#pragma unroll 1
+    for (int round = 0; round < kInvMaxRounds; ++round) {
+        int32_t any = 0;
+#pragma unroll
+        for (int i = 0; i < kInvLimbs; ++i) any |= g[i];
+        if (any == 0) break;
+        // thirty steps on the low words: 2^i f_i = u f + v g, 2^i g_i = q f + r g
+        int32_t u = 1, v = 0, q = 0, r = 1;
+        uint32_t f0 = (uint32_t)f[0] | ((uint32_t)f[1] << kInvBits), g0 = (uint32_t)g[0] | ((uint32_t)g[1] << kInvBits);
+#pragma unroll 6
+        for (int i = 0; i < kInvBits; ++i) {
+            const bool odd = g0 & 1u, swap = odd && delta > 0;
+            const uint32_t af = odd ? (swap ? 0u - f0 : f0) : 0u;
+            const int32_t au = odd ? (swap ? -u : u) : 0, av = odd ? (swap ? -v : v) : 0;
+            delta = 2 + (swap ? -delta : delta);
+            f0 = swap ? g0 : f0;
+            u = (swap ? q : u) << 1;
+            v = (swap ? r : v) << 1;
+            g0 = (g0 + af) >> 1;
+            q += au;
+            r += av;
+        }
+        // f, g = (u f + v g) / 2^30, (q f + r g) / 2^30: the low thirty bits are zero
+        int64_t cf = (int64_t)u * f[0] + (int64_t)v * g[0], cg = (int64_t)q * f[0] + (int64_t)r * g[0];
+        // d, e likewise, with m p added for the m < 2^30 that clears the low limb:
+        // |u| + |v| <= 2^30, so |d| and |e| grow by less than p a round
+        int64_t cd = (int64_t)u * d[0] + (int64_t)v * e[0], ce = (int64_t)q * d[0] + (int64_t)r * e[0];
+        const int32_t md = (int32_t)((uint32_t)cd * BLS_NINV) & kInvMask, me = (int32_t)((uint32_t)ce * BLS_NINV) & kInvMask;
+        cd += (int64_t)md * P30[0];
+        ce += (int64_t)me * P30[0];
+        cf >>= kInvBits;
+        cg >>= kInvBits;
+        cd >>= kInvBits;
+        ce >>= kInvBits;
+#pragma unroll
+        for (int i = 1; i < kInvLimbs; ++i) {
+            cf += (int64_t)u * f[i] + (int64_t)v * g[i];
+            cg += (int64_t)q * f[i] + (int64_t)r * g[i];
+            cd += (int64_t)u * d[i] + (int64_t)v * e[i] + (int64_t)md * P30[i];
+            ce += (int64_t)q * d[i] + (int64_t)r * e[i] + (int64_t)me * P30[i];
+            f[i - 1] = (int32_t)cf & kInvMask;
+            g[i - 1] = (int32_t)cg & kInvMask;
+            d[i - 1] = (int32_t)cd & kInvMask;
+            e[i - 1] = (int32_t)ce & kInvMask;
+            cf >>= kInvBits;
+            cg >>= kInvBits;
+            cd >>= kInvBits;
+            ce >>= kInvBits;
+        }
+        f[kInvLimbs - 1] = (int32_t)cf;
+        g[kInvLimbs - 1] = (int32_t)cg;
+        d[kInvLimbs - 1] = (int32_t)cd;
+        e[kInvLimbs - 1] = (int32_t)ce;
+    }
+    // f = +-1 and d x = f: |d| < 37 p, the limbs below the top one nonnegative.
+    // +-d + 64 p, in 32-bit words, then the multiples of p off.
+    const bool neg = f[kInvLimbs - 1] < 0;
+    int64_t c = 0;
+    uint64_t acc = 0;
+    int bits = 0, k = 0;
+#pragma unroll
+    for (int i = 0; i < kInvLimbs; ++i) {
+        c += (neg ? -(int64_t)d[i] : (int64_t)d[i]) + 64 * (int64_t)P30[i];
+        const uint64_t limb = i == kInvLimbs - 1 ? (uint64_t)c : (uint64_t)(c & kInvMask);
+        c >>= kInvBits;
+        acc |= limb << bits;
+        bits += kInvBits;
+        if (bits >= 32) {
+            t[k++] = (uint32_t)acc;
+            acc >>= 32;
+            bits -= 32;
+        }
+    }
+    t[12] = (uint32_t)acc;
+#pragma unroll
+    for (int j = 6; j >= 0; --j) {      // below 2^(j+1) p: 2^j p off when it fits
+        uint32_t w[13], br = 0;
+#pragma unroll
+        for (int i = 0; i < 13; ++i) {
+            const uint32_t lo = i < 12 ? P_[i] << j : 0u, hi = (i > 0 && j > 0) ? P_[i - 1] >> (32 - j) : 0u;
+            const uint64_t y = (uint64_t)t[i] - (lo | hi) - br;
+            w[i] = (uint32_t)y;
+            br = (uint32_t)(y >> 63);
+        }
+#pragma unroll
+        for (int i = 0; i < 13; ++i) t[i] = br ? t[i] : w[i];
+    }
+    fp inv, r3;
 #pragma unroll
     for (int i = 0; i < 12; ++i) {
-        u[i] = x.w[i];
-        v[i] = P_[i];
-        x1[i] = 0;
-        x2[i] = 0;
+        inv.w[i] = t[i];
+        r3.w[i] = kR3[i];
     }
-    x1[0] = 1;
-    // u, v stay odd-or-positive and gcd(u, v) = 1; every pass of the outer
-    // loop removes at least one bit from u or v, so 2 * 381 + 2 passes end it
-    for (int iter = 0; iter < 800 && !u_is_one(u) && !u_is_one(v); ++iter) {
-        for (int k = 0; k < 384 && (u[0] & 1u) == 0; ++k) {
-            shr1(u);
-            half_mod(x1);
-        }
-        for (int k = 0; k < 384 && (v[0] & 1u) == 0; ++k) {
-            shr1(v);
-            half_mod(x2);
-        }
-        if (geq12(u, v)) {
-            sub12(u, v);
-            sub_mod(x1, x2);
-        } else {
-            sub12(v, u);
-            sub_mod(x2, x1);
-        }
-    }
-    fp r;
-    const bool uone = u_is_one(u);
-#pragma unroll
-    for (int i = 0; i < 12; ++i) r.w[i] = uone ? x1[i] : x2[i];
-    fp r3;
-#pragma unroll
-    for (int i = 0; i < 12; ++i) r3.w[i] = kR3[i];
-    return fp_mul(r, r3);                              // r R^3 / R: Montgomery form of a^-1
-}
-
-
-__device__ __forceinline__ fp shfl_fp(const fp& v, int src) {
-    fp r;
-#pragma unroll
-    for (int i = 0; i < 12; ++i) r.w[i] = __shfl_sync(0xffffffffu, v.w[i], src);
-    return r;
-}
-__device__ __forceinline__ fp shfl_up_fp(const fp& v, int d) {
-    fp r;
-#pragma unroll
-    for (int i = 0; i < 12; ++i) r.w[i] = __shfl_up_sync(0xffffffffu, v.w[i], d);
-    return r;
-}
-__device__ __forceinline__ fp shfl_down_fp(const fp& v, int d) {
-    fp r;
-#pragma unroll
-    for (int i = 0; i < 12; ++i) r.w[i] = __shfl_down_sync(0xffffffffu, v.w[i], d);
-    return r;
-}
-
-// The Fp inverses of the 32 lanes' values by Montgomery's simultaneous-
-// inversion trick over the warp: prefix and suffix products by shuffles (five
-// multiplications each), one inverse of the whole product, which every lane
-// computes from the same value so the binary Euclid's data-dependent branches
-// never split the warp, and two multiplications per lane.  Each lane's own
-// binary Euclid on its own value would diverge and serialise the warp's 32
-// paths.  Every lane of the warp must call it together (full-mask shuffles).
-// z: any value below 2^381 + p; 0 gives 0, as fp_inverse_mont does (a zero
-// stands in as one in the products); kR3: R^3 mod p.
-static __device__ __noinline__ fp fp_inverse_warp(fp z, const uint32_t* kR3) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {          // canonical: fp_mul wants inputs below p
-        uint32_t d[12];
-        const uint32_t br = sub_p(d, z.w);
-#pragma unroll
-        for (int i = 0; i < 12; ++i) z.w[i] = br ? z.w[i] : d[i];
-    }
-    const bool zero = fp_is_zero(z);
-    const fp x = zero ? fp_one() : z;
-    fp pre = x, suf = x;                    // inclusive prefix and suffix products
-    for (int d = 1; d < 32; d <<= 1) {
-        const fp y = shfl_up_fp(pre, d);
-        if (lane >= d) pre = fp_mul_ool(y, pre);
-    }
-    for (int d = 1; d < 32; d <<= 1) {
-        const fp y = shfl_down_fp(suf, d);
-        if (lane + d < 32) suf = fp_mul_ool(suf, y);
-    }
-    const fp total = shfl_fp(pre, 31);
-    fp before = shfl_up_fp(pre, 1), after = shfl_down_fp(suf, 1);
-    if (lane == 0) before = fp_one();
-    if (lane == 31) after = fp_one();
-    const fp t = fp_inverse_mont(total, kR3);
-    const fp r = fp_mul_ool(fp_mul_ool(t, before), after);
-    return zero ? fp_zero() : r;
+    return fp_mul(inv, r3);             // x^-1 R^3 / R: the Montgomery form of a^-1
 }
 
 }  // namespace bls

@@ -40,14 +40,11 @@ __global__ void __launch_bounds__(kHashThreads) k_neg_hash_to_g1(const uint8_t* 
         }
     }
     __syncthreads();
-    // the even thread of a live message adds the points and clears the
-    // cofactor; then every thread of the warp takes part in one simultaneous
-    // inversion of the results' Z (the others contribute a one), so the
-    // warp's 16 inverses cost one binary Euclid that does not diverge
-    const bool owner = live && !which;
+    // the even thread of a live message adds the points, clears the cofactor
+    // and inverts the result's Z
+    if (!live || which) return;
     g1j r;
-    r.Z = fp_one();
-    if (owner) {
+    {
         const uint4* d = xch[threadIdx.x >> 1];
         g1j p1;
         fp* c[3] = {&p1.X, &p1.Y, &p1.Z};
@@ -60,8 +57,7 @@ __global__ void __launch_bounds__(kHashThreads) k_neg_hash_to_g1(const uint8_t* 
             }
         r = h2c::clear_sum(pt, p1);
     }
-    const fp zi = fp_inverse_warp(owner ? r.Z : fp_one(), h2c::kR3);
-    if (!owner) return;
+    const fp zi = fp_inverse_mont(r.Z, h2c::kR3);
     fp ox, oy;
     h2c::neg_affine(r, zi, ox, oy);
     fp_store_u64(out + 12 * (size_t)i, ox);

@@ -5,7 +5,7 @@
 // Formulas follow the reference tower (gpu-crypto/cuda/field_sppark.cuh:52-197),
 // which mirrors ic_bls12_381 0.10.1: Karatsuba Fp2/Fp6/Fp12 products, the sparse
 // line product mul_by_014, Frobenius with fixed Montgomery constants, the
-// inversion (binary extended Euclid, fp_inv.cuh; the reference's Fermat power
+// inversion (division steps, fp_inv.cuh; the reference's Fermat power
 // gives the same value), and Granger-Scott squaring in the cyclotomic
 // subgroup.  The tower keeps its products inline: the out-of-line multiply of
 // fp.cuh made the thread-per-verification kernel 20% faster but the key
@@ -51,7 +51,7 @@ static __device__ __noinline__ fp2 fp2_sqr(const fp2& a) {
 }
 
 // a^-1, 0 for 0 (the reference's Fermat a^(p-2), field_sppark.cuh:40-50,
-// gives the same value): the binary extended Euclid of fp_inv.cuh
+// gives the same value): the division steps of fp_inv.cuh
 static __device__ __noinline__ fp fp_inv(const fp& a) {
     const fp r3 = fp_mul(fp_rr(), fp_rr());              // R^3 mod p
     return fp_inverse_mont(a, r3.w);

@@ -14,7 +14,7 @@
 //                 LINE1 and LINE2 multiply f by the two lines; 62 SQR in
 //                 between; CONJ at the end (x < 0)
 //   final exp     the reference's chain over 7 Fp12 groups, the inverse in 8
-//                 steps with an extended-Euclid Fp inverse on one thread
+//                 steps with an Fp inverse on one thread
 //   result        canonical Gt compared with 1; optional Miller / Gt outputs
 //
 // Shared memory: 8 block-shared constant slots (0, 1, Frobenius constants),

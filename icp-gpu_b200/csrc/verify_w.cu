@@ -291,12 +291,12 @@ __device__ __forceinline__ void run(int pid, const Sm& s, int k, int half, const
         const uint32_t nl = (hdr >> 4) & 3u, scale = (hdr >> 6) & 3u, bias = (hdr >> 16) & 0xffu;
         const uint32_t* lin = f2::kPair + off + 2 + np;
         uint32_t o[12];
-        if ((hdr >> 24) & 1u) {                     // the one Fp inverse, all 32 items together
+        if ((hdr >> 24) & 1u) {                     // the one Fp inverse
             fp r = fp_zero();
             if (half == 0) {
                 fp z;
                 load_fp(z.w, s, slot_addr(bs, lin[0] >> 8), 0);
-                r = fp_inverse_warp(z, f2::kR3);
+                r = fp_inverse_mont(z, f2::kR3);
             }
 #pragma unroll
             for (int i = 0; i < 12; ++i) o[i] = r.w[i];
