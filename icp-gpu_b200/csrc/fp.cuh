@@ -514,13 +514,13 @@ __device__ __forceinline__ void sqr_row(uint32_t* A, uint32_t* B, const uint32_t
     }
 }
 
-// Montgomery square a^2 R^-1 mod p for a < 2p, canonical (below p): row i takes
+// Montgomery square a^2 R^-1 mod p for a <= 3p, canonical (below p): row i takes
 // a_i times a_i and times the limbs above it of 2a (whose lowest, a_{i+1}, enters
 // without the bit that belongs to a_i), so the 66 cross products are formed once:
 // 78 paired multiply-adds, in the two column vectors of the file comment.  Then the
 // low twelve limbs are Montgomery-reduced on their own, (t_lo + m p) / R <= p,
-// and the high twelve added: a^2 / R + p < 1.5p for a < 2p, so one conditional
-// subtraction ends it.  222 paired multiply-adds where the general product takes
+// and the high twelve added: a^2 / R + p < 1.92p for a <= 3p (p / R < 0.1017), so one
+// conditional subtraction ends it.  222 paired multiply-adds where the general product takes
 // 288; the same value as fp_mul(a, a).
 __device__ __forceinline__ fp fp_sqr(const fp& a) {
     uint32_t A[24], B[24], d[12];
@@ -621,6 +621,27 @@ __device__ __forceinline__ fp fp_add(const fp& a, const fp& b) {
     fp r;
 #pragma unroll
     for (int i = 0; i < 12; ++i) r.w[i] = s[i];
+    return r;
+}
+
+// a + b without the range reduction: below 2^384 while the sum is below 9p
+__device__ __forceinline__ fp fp_add_nr(const fp& a, const fp& b) {
+    fp r;
+    asm("add.cc.u32 %0, %12, %24;\n\t"
+        "addc.cc.u32 %1, %13, %25;\n\t"
+        "addc.cc.u32 %2, %14, %26;\n\t"
+        "addc.cc.u32 %3, %15, %27;\n\t"
+        "addc.cc.u32 %4, %16, %28;\n\t"
+        "addc.cc.u32 %5, %17, %29;\n\t"
+        "addc.cc.u32 %6, %18, %30;\n\t"
+        "addc.cc.u32 %7, %19, %31;\n\t"
+        "addc.cc.u32 %8, %20, %32;\n\t"
+        "addc.cc.u32 %9, %21, %33;\n\t"
+        "addc.cc.u32 %10, %22, %34;\n\t"
+        "addc.u32 %11, %23, %35;"
+        : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]), "=r"(r.w[5]), "=r"(r.w[6]),
+          "=r"(r.w[7]), "=r"(r.w[8]), "=r"(r.w[9]), "=r"(r.w[10]), "=r"(r.w[11])
+        : BLS_A12(a.w), BLS_A12(b.w));
     return r;
 }
 

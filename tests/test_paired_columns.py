@@ -96,8 +96,8 @@ def test_rows_at_the_ends_of_their_ranges():
     for t in EDGES + [R - 1, R - 2, (R - 1) // M32]:
         v = mont(0, t=t)
         assert (v * R - t) % P == 0 and v <= P
-    for a in [v for v in EDGES if v < 2 * P]:
-        assert sqr_columns(a) == a * a
+    for a in [v for v in EDGES if v < 2 * P] + [3 * P, 3 * P - 1]:
+        assert sqr_columns(a) == a * a and a * a // R + P < 2 * P
 
 
 @pytest.mark.gpu
