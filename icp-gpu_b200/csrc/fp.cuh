@@ -740,7 +740,9 @@ static __device__ __noinline__ fp fp_sqr_ool(const fp& a) { return fp_sqr(a); }
 // a left-to-right sliding window of four bits over the odd powers a, a^3, ...,
 // a^15: one squaring per bit and one product per window, about nbits / 5 of
 // them, where the bit-by-bit power takes one product per set bit.  a below
-// 2p; the result is canonical (a^0 = 1, 0^e = 0 for e > 0).
+// 2p; the result is canonical (a^0 = 1, 0^e = 0 for e > 0).  The squaring is inlined
+// at its one place, a loop of its own: a call passes its operands through local
+// memory.
 __device__ __forceinline__ fp fp_pow_ool(const fp& a, const uint64_t* e, int nbits) {
     fp odd[8];
     odd[0] = a;
@@ -749,21 +751,27 @@ __device__ __forceinline__ fp fp_pow_ool(const fp& a, const uint64_t* e, int nbi
     auto bit = [&](int i) { return (int)((e[i >> 6] >> (i & 63)) & 1u); };
     fp r = fp_one();
     bool started = false;
+#pragma unroll 1
     for (int i = nbits - 1; i >= 0;) {
-        if (!bit(i)) {
-            if (started) r = fp_sqr_ool(r);
-            --i;
-            continue;
-        }
-        int j = i >= 3 ? i - 3 : 0;                  // the window [j, i] ends on a set bit
-        while (!bit(j)) ++j;
+        int j = i;                                   // squarings down to bit j, and the window's value
+        while (j >= 0 && !bit(j)) --j;
         int v = 0;
-        for (int k = i; k >= j; --k) {
-            v = (v << 1) | bit(k);
-            if (started) r = fp_sqr_ool(r);
+        if (j >= 0) {                                // the window [w, j] ends on a set bit
+            int w = j >= 3 ? j - 3 : 0;
+            while (!bit(w)) ++w;
+            for (int k = j; k >= w; --k) v = (v << 1) | bit(k);
+            j = w;
+        } else {
+            j = 0;
         }
-        r = started ? fp_mul_ool(r, odd[v >> 1]) : odd[v >> 1];
-        started = true;
+        if (started) {
+#pragma unroll 1
+            for (int k = i; k >= j; --k) r = fp_sqr(r);
+            if (v) r = fp_mul(r, odd[v >> 1]);
+        } else if (v) {
+            r = odd[v >> 1];
+            started = true;
+        }
         i = j - 1;
     }
     return r;

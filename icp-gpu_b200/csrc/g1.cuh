@@ -223,6 +223,39 @@ static __device__ __noinline__ g1j quad_add_affine(const g1j& p, const fp& qx, c
     return r;
 }
 
+// p + q, both Jacobian (add-2007-bl with Z3 = 2 Z1 Z2 H); *bad as for quad_add_affine
+static __device__ __noinline__ g1j quad_add(const g1j& p, const g1j& q, bool* bad) {
+    const int l = threadIdx.x & 3;
+    const bool odd = l & 1, high = l >> 1;
+    // Z1^2, Z2^2, Y1 Z2, Y2 Z1
+    fp s = fp_mul_ool(fp_sel(high, fp_sel(odd, q.Y, p.Y), fp_sel(odd, q.Z, p.Z)), fp_sel(l == 0 || l == 3, p.Z, q.Z));
+    const fp ZZ1 = quad_get(s, 0), ZZ2 = quad_get(s, 1), YZ1 = quad_get(s, 2), YZ2 = quad_get(s, 3);
+    // U1, U2, S1, S2
+    s = fp_mul_ool(fp_sel(high, fp_sel(odd, YZ2, YZ1), fp_sel(odd, q.X, p.X)), fp_sel(odd, ZZ1, ZZ2));
+    const fp U1 = quad_get(s, 0), S1 = quad_get(s, 2);
+    const fp H = fp_sub(quad_get(s, 1), U1);
+    fp rr = fp_sub(quad_get(s, 3), S1);
+    rr = fp_add(rr, rr);
+    if (fp_is_zero(p.Z) || fp_is_zero(q.Z) || fp_is_zero(H)) *bad = true;
+    // (2H)^2, rr^2, Z1 Z2
+    fp I = fp_add(H, H);
+    s = fp_mul_ool(fp_sel(high, p.Z, fp_sel(odd, rr, I)), fp_sel(high, q.Z, fp_sel(odd, rr, I)));
+    I = quad_get(s, 0);
+    const fp rr2 = quad_get(s, 1), zz = quad_get(s, 2);
+    // J = H I, V = U1 I, Z1 Z2 H
+    s = fp_mul_ool(fp_sel(high, zz, fp_sel(odd, U1, H)), fp_sel(high, H, I));
+    const fp J = quad_get(s, 0), V = quad_get(s, 1);
+    g1j r;
+    r.Z = quad_get(s, 2);
+    r.Z = fp_add(r.Z, r.Z);
+    r.X = fp_sub(fp_sub(rr2, J), fp_add(V, V));
+    // rr (V - X3), S1 J
+    s = fp_mul_ool(fp_sel(odd, S1, rr), fp_sel(odd, J, fp_sub(V, r.X)));
+    const fp SJ = quad_get(s, 1);
+    r.Y = fp_sub(quad_get(s, 0), fp_add(SJ, SJ));
+    return r;
+}
+
 // g1_in_subgroup with four lanes to the point
 static __device__ __noinline__ bool quad_in_subgroup(const fp& x, const fp& y) {
     const uint64_t k[2] = {0x0000000100000000ULL, 0xac45a4010001a402ULL};

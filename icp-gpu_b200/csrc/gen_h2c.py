@@ -346,6 +346,18 @@ def emit():
         fparr(name, [v])
     arr("kSqrtRatioE", limbs64(SQRT_RATIO_E), "0x%016xull", "uint64_t")
     L.append("constexpr int kSqrtRatioBits = %d;  // (p - 3) / 4" % SQRT_RATIO_E.bit_length())
+    L.append("// the 11-isogeny E' -> E as four polynomials of degree 15 (x numerator, x denominator, y numerator,")
+    L.append("// y denominator; zeros above their own degree): kIsoQuad[degree][polynomial]")
+    L.append("#ifndef BLS_H2C_TABLE")
+    L.append("#define BLS_H2C_TABLE BLS_H2C_CONST")
+    L.append("#endif")
+    quad = [ISO_X_NUM, ISO_X_DEN, ISO_Y_NUM, ISO_Y_DEN]
+    assert max(map(len, quad)) == 16
+    L.append("BLS_H2C_TABLE uint64_t kIsoQuad[16][4][6] = {")
+    for i in range(16):
+        L.append("    {" + ", ".join("{" + ", ".join("0x%016xull" % v for v in mont(c[i] if i < len(c) else 0)) + "}"
+                                      for c in quad) + "},")
+    L.append("};")
     L.append("// the 11-isogeny E' -> E: coefficients by degree; the denominators are monic")
     L.append("// (leading 1 not stored): x = x_num / x_den, y = y' y_num / y_den")
     fparr("kIsoXNum", ISO_X_NUM)
