@@ -1035,6 +1035,47 @@ def line_pair(k):
     return d
 
 
+def split_products(c, h, lanes):
+    """The products of warp h dealt to `lanes` lanes of an item (a power of two): a
+    list per lane, run side by side and summed at the end.  A stored partial sum is
+    the work of one lane alone, which begins with it."""
+    segs, own, cur, done = [], [], [], 0
+    for i, p in enumerate(c.prods[h]):
+        cur.append(p[:4])
+        if p[4]:
+            segs.append([q + (None,) for q in cur[:-1]] + [cur[-1] + (("sum", p[4][1]),)])
+            cur, done = [], i + 1
+    own = [p[:4] + (None,) for p in c.prods[h][done:]]
+    assert len(segs) <= lanes and all(p[4] is None for p in c.prods[h][done:])
+    lists = segs + [[] for _ in range(lanes - len(segs))]
+    for p in own:
+        min(lists, key=len).append(p)
+    return lists
+
+
+def encode_product(p):
+    uf, ur, vf, vr, store = p
+    combo = COMBO_LINE if uf == X_LINE else COMBOS.index((uf, vf)) if (uf, vf) in COMBOS else COMBO_GENERIC
+    assert combo not in (4,) or ur == vr        # (x0 + x1)(x0 - x1): one slot
+    x = combo | (vf << 4) | (ur << 8) | (vr << 16)
+    x |= ((uf & 1) << 15) | ((uf >> 1 & 1) << 23) | ((uf >> 2 & 1) << 30) | ((uf >> 3 & 1) << 31)
+    if store:
+        assert store[1] < PART_SLOTS
+        x |= ((1 if store[0] == "sum" else 2) << 24) | (store[1] << 26)
+    assert x != NO_PRODUCT
+    return x
+
+
+NO_PRODUCT = 0xffffffff     # a lane without a product at a step
+
+
+def encode_split(c, h, lanes):
+    """steps, then per step the word of each lane"""
+    lists = split_products(c, h, lanes)
+    steps = max(map(len, lists))
+    return [steps] + [encode_product(q[i]) if i < len(q) else NO_PRODUCT for i in range(steps) for q in lists]
+
+
 def encode_pair(c, h):
     """the descriptor of warp h: header products | linear terms << 4 | scale << 6 | dst << 8 | bias << 16 |
     inverse << 24; the two added slots, a byte each (15: none, and ends the list; 16 set: subtracted); then products combo (COMBOS) | vform << 4 | uref << 8 | vref << 16 | store << 24 (1: sum,
@@ -1045,15 +1086,7 @@ def encode_pair(c, h):
          (int(c.invfp) << 24)]
     adds = [sl | (16 if sign < 0 else 0) for sl, sign in c.adds[h]] + [15, 15]
     w.append(adds[0] | (adds[1] << 8) | (15 << 16))
-    for uf, ur, vf, vr, store in c.prods[h]:
-        combo = COMBO_LINE if uf == X_LINE else COMBOS.index((uf, vf)) if (uf, vf) in COMBOS else COMBO_GENERIC
-        assert combo not in (4,) or ur == vr        # (x0 + x1)(x0 - x1): one slot
-        x = combo | (vf << 4) | (ur << 8) | (vr << 16)
-        x |= ((uf & 1) << 15) | ((uf >> 1 & 1) << 23) | ((uf >> 2 & 1) << 30) | ((uf >> 3 & 1) << 31)
-        if store:
-            assert store[1] < PART_SLOTS
-            x |= ((1 if store[0] == "sum" else 2) << 24) | (store[1] << 26)
-        w.append(x)
+    w += [encode_product(p) for p in c.prods[h]]
     return w + [(co & 15) | (r << 8) for co, r in c.lins[h]]
 
 
@@ -1175,6 +1208,24 @@ def emit(path):
         L.append("    {%s}," % ", ".join("%d" % v for v in row))
     L.append("};")
     L.append("constexpr int kPartSlots = %d;" % PART_SLOTS)
+    L.append("constexpr uint32_t kNoProduct = 0x%08xu;" % NO_PRODUCT)
+    for lanes in (2, 4):
+        sw, si = [], []
+        for row in [pairs(outs) for _, outs, _ in progs] + [[line_pair(k) for k in range(6)]]:
+            si.append([])
+            for h in range(2):
+                for c in row:
+                    si[-1].append(len(sw))
+                    sw += encode_split(c, h, lanes) if c is not None else [0]
+        L.append("// the same products dealt to %d lanes of an item: steps, then a word per step and lane" % lanes)
+        L.append("__device__ __constant__ uint16_t kSplit%dIndex[%d][12] = {" % (lanes, len(si)))
+        for row in si:
+            L.append("    {%s}," % ", ".join("%d" % v for v in row))
+        L.append("};")
+        L.append("__device__ __constant__ uint32_t kSplit%d[%d] = {" % (lanes, len(sw)))
+        for i in range(0, len(sw), 6):
+            L.append("    " + ", ".join("0x%08xu" % w for w in sw[i:i + 6]) + ",")
+        L.append("};")
     L.append("__device__ __constant__ uint32_t kPair[%d] = {" % len(words))
     for i in range(0, len(words), 6):
         L.append("    " + ", ".join("0x%08xu" % w for w in words[i:i + 6]) + ",")

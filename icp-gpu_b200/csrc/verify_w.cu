@@ -40,7 +40,7 @@
 namespace bls {
 namespace {
 
-constexpr int kV = 32;                           // items per block, one per lane
+constexpr int kV = 32;                           // items a block holds at most, one per lane
 constexpr int kRoles = 12;                       // warps per block
 constexpr int kThreads = 32 * kRoles;
 constexpr int kGroups = f2::kGroupsUsed;
@@ -49,12 +49,14 @@ constexpr int kCOff = 6 * kGroups;               // C area after the groups
 constexpr int kItemSlots = kCOff + 12;           // Fp2 slots per item
 constexpr int kSlotU4 = kItemSlots * 6 * kV;     // 16-byte units of the item slots
 constexpr int kKU4 = kKSlots * 6;                // constant slots, not interleaved
-constexpr int kXchU4 = f2::kPartSlots * 7 * kV;  // partial sums: 25 words (7 units) per slot and item
+constexpr int kXchU4 = 6 * 2 * 7 * kV;           // partial sums: 25 words (7 units) per coefficient, half, item
+constexpr int kXchAntiU4 = 3 * 7 * kV;           // and the square's subtracted sums, of three coefficients
+static_assert((kXchU4 + kXchAntiU4) / (7 * kV) == f2::kPartSlots, "a slot of 7 units per partial sum and item");
 constexpr int kKpCount = f2::kMaxBias + 1;       // k p, 16 words each
 constexpr int kInfoWords = 4 * kV;               // per item: key index, flags, status, result flags
 constexpr int kFlagBytes = 16 * kV;              // per item and role: "not the expected value" bytes
 constexpr int kQpU4 = 128 * 4;                   // the QP table (128 entries of 16 words)
-constexpr size_t kSmemBytes = (size_t)(kSlotU4 + kKU4 + kXchU4 + kQpU4) * 16 + (size_t)kKpCount * 64 +
+constexpr size_t kSmemBytes = (size_t)(kSlotU4 + kKU4 + kXchU4 + kXchAntiU4 + kQpU4) * 16 + (size_t)kKpCount * 64 +
                               (size_t)kInfoWords * 4 + kFlagBytes + 16;
 static_assert(kKSlots + kItemSlots <= 256, "slot indices must fit a byte");
 static_assert(kKpCount <= kThreads, "one thread per table entry at start-up");
@@ -272,18 +274,58 @@ __device__ __forceinline__ void sum_products(uint32_t* acc, const uint32_t* prod
     }
 }
 
+// The same with kSplit lanes to an item: each lane sums its list of the products
+// (gen_fp2ops.py: split_products), and the lanes' sums are added at the end, in
+// every lane.
+template <int kSplit>
+__device__ __forceinline__ void sum_products_split(uint32_t* acc, const uint32_t* list, const Sm& s, const Bases& bs,
+                                                   const uint32_t* line) {
+    constexpr int kItems = kV / kSplit;
+    const int sub = (threadIdx.x & 31) / kItems;
+    const uint32_t steps = list[0];
+#pragma unroll
+    for (int i = 0; i < 25; ++i) acc[i] = 0;
+#pragma unroll 1
+    for (uint32_t j = 0; j < steps; ++j) {
+        const uint32_t w = list[1 + kSplit * j + sub];
+        if (w != f2::kNoProduct) {
+            uint32_t U[12], V[12], P[24];
+            load_operands(U, V, s, w, bs, line);
+            f2::prod24k(P, U, V);
+            f2::add25(acc, P);
+            if ((w >> 24) & 3u) part_store(part_row(s, (w >> 26) & 15u), acc, acc[24]);
+        }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int d = kItems; d < kV; d *= 2) {
+        uint32_t p[25];
+#pragma unroll
+        for (int i = 0; i < 25; ++i) p[i] = __shfl_xor_sync(0xffffffffu, acc[i], d);
+        f2::add25_25(acc, p);
+    }
+}
+
 // Warp (k, half) on program `pid` for every item of the block.  No program of
 // the generated sequences writes a slot that any warp of it reads (the
 // generator places a result that would overwrite an operand in an unused group,
 // and refuses to emit a sequence where it cannot), so a warp stores its
 // component as soon as it has it: one block-wide meeting per program, after the
 // stores, and one of a coefficient's two warps when the partial sums are there.
+template <int kSplit>
 __device__ __forceinline__ void run(int pid, const Sm& s, int k, int half, const Bases& bs, const uint32_t* line) {
     const uint32_t off = f2::kPairIndex[pid][6 * half + k];
     const uint32_t hdr = off != 0xffffu ? f2::kPair[off] : 0u, adds = off != 0xffffu ? f2::kPair[off + 1] : 0u;
     const uint32_t np = hdr & 15u;
     uint32_t acc[25];
-    if (np) sum_products(acc, f2::kPair + off + 2, np, s, bs, line);
+    if (np) {
+        if constexpr (kSplit == 1)
+            sum_products(acc, f2::kPair + off + 2, np, s, bs, line);
+        else if constexpr (kSplit == 2)
+            sum_products_split<2>(acc, f2::kSplit2 + f2::kSplit2Index[pid][6 * half + k], s, bs, line);
+        else
+            sum_products_split<4>(acc, f2::kSplit4 + f2::kSplit4Index[pid][6 * half + k], s, bs, line);
+    }
     // a named barrier (id 1 + k) over the 64 threads of coefficient k; both
     // warps reach it on every program, whether or not they have an output
     asm volatile("bar.sync %0, 64;" ::"r"(1 + k) : "memory");
@@ -447,13 +489,18 @@ __device__ bool serve_claim(const VerifyArgs& a, uint64_t t_launch, uint32_t* ba
     return false;
 }
 
+// kSplit lanes work on each item, 32 / kSplit items a block.  What a block does
+// takes the same time whether its lanes hold 32 items or one, so a batch that
+// would leave lanes empty gives them a share of the products instead.
+template <int kSplit>
 __global__ void __launch_bounds__(kThreads, 1) k_verify_w(VerifyArgs a, const uint32_t* __restrict__ in_status) {
+    constexpr int kItems = kV / kSplit;
     extern __shared__ uint4 smem4[];
     Sm s;
     s.slots = smem4;
     s.kslots = smem4 + kSlotU4;
     s.xch = s.kslots + kKU4;
-    s.qp = s.xch + kXchU4;
+    s.qp = s.xch + kXchU4 + kXchAntiU4;
     s.kp = reinterpret_cast<uint32_t*>(s.qp + kQpU4);
     s.info = s.kp + 16 * kKpCount;
     s.flags = reinterpret_cast<uint8_t*>(s.info + kInfoWords);
@@ -462,7 +509,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_verify_w(VerifyArgs a, const ui
     // descriptor decoding and branches on uniform registers (3.75 -> 3.65 ms)
     const int role = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
     const int half = role / 6, k = role % 6;
-    s.v = threadIdx.x & 31;
+    s.v = threadIdx.x & (kItems - 1);
+    const bool lead = (threadIdx.x & 31) < kItems;   // of an item's lanes, the one that writes results
 
     {
         uint32_t* kw = reinterpret_cast<uint32_t*>(s.kslots);
@@ -490,8 +538,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_verify_w(VerifyArgs a, const ui
     const uint64_t* g2_lines = norm ? a.g2_norm : a.g2;
     const bool serving = a.serve_avail != nullptr;
     const uint64_t t_launch = serving ? globaltimer_ns() : 0;
-    int next = blockIdx.x * kV;
-    const int stride = gridDim.x * kV;
+    int next = blockIdx.x * kItems;
+    const int stride = gridDim.x * kItems;
     uint32_t* info = s.info + 4 * s.v;
 
     for (;;) {
@@ -510,7 +558,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_verify_w(VerifyArgs a, const ui
             if (count == 0) break;
         } else {
             if (a.work_counter) {
-                if (threadIdx.x == 0) s.bcast[0] = (uint32_t)atomicAdd(a.work_counter, kV);
+                if (threadIdx.x == 0) s.bcast[0] = (uint32_t)atomicAdd(a.work_counter, kItems);
                 __syncthreads();
                 base = (int)s.bcast[0];
                 __syncthreads();
@@ -519,7 +567,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_verify_w(VerifyArgs a, const ui
                 next += stride;
             }
             if (base >= a.n) break;
-            count = a.n - base < kV ? a.n - base : kV;
+            count = a.n - base < kItems ? a.n - base : kItems;
         }
         const bool have = s.v < count;
         // item = ring slot (serving) or batch index
@@ -597,7 +645,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_verify_w(VerifyArgs a, const ui
                 ++st;
             }
             if (code < (uint32_t)f2::kNumPrograms || code == f2::kOpLoadLines) {
-                run(pid, s, k, half, bs, line);
+                run<kSplit>(pid, s, k, half, bs, line);
             } else if (code == f2::kOpLoadCorr) {
                 // the generator's and the key's Miller correction factors into the c2 slots
                 if (k < 2) {
@@ -607,12 +655,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_verify_w(VerifyArgs a, const ui
                 }
                 __syncthreads();
             } else if (code == f2::kOpMillerDone) {
-                if (a.ml_out) emit_group(s, (e >> 5) & 7u, k, half, have ? a.ml_out + 72 * (size_t)item : nullptr);
+                if (a.ml_out) emit_group(s, (e >> 5) & 7u, k, half, have && lead ? a.ml_out + 72 * (size_t)item : nullptr);
             }
         }
         const bool one = emit_group(s, (int)f2::kGtGroup[norm], k, half,
-                                    (have && a.gt_out) ? a.gt_out + 72 * (size_t)item : nullptr);
-        if (have && role == 0) {
+                                    (have && lead && a.gt_out) ? a.gt_out + 72 * (size_t)item : nullptr);
+        if (have && lead && role == 0) {
             const int32_t status = (int32_t)info[2];
             a.results[item] = status != 0 ? -status : (one ? 1 : 0);
         }
@@ -621,8 +669,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_verify_w(VerifyArgs a, const ui
 }
 
 cudaError_t configure() {
-    static cudaError_t done =
-        cudaFuncSetAttribute(k_verify_w, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+    static cudaError_t done = [] {
+        cudaError_t e = cudaSuccess;
+        for (const void* f : {(const void*)k_verify_w<1>, (const void*)k_verify_w<2>, (const void*)k_verify_w<4>})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+        return e;
+    }();
     return done;
 }
 
@@ -633,7 +685,7 @@ size_t verify_w_smem_bytes() { return kSmemBytes; }
 int verify_w_blocks_per_sm() {
     if (configure() != cudaSuccess) return 0;
     int blocks = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_verify_w, kThreads, kSmemBytes) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_verify_w<1>, kThreads, kSmemBytes) != cudaSuccess)
         return 0;
     return blocks;
 }
@@ -646,19 +698,67 @@ cudaError_t launch_verify_w_serve(const VerifyArgs& a, const uint32_t* in_status
     cudaError_t e = configure();
     if (e != cudaSuccess) return e;
     if (blocks > sms) blocks = sms;
-    k_verify_w<<<blocks, kThreads, kSmemBytes, s>>>(a, in_status);
+    k_verify_w<1><<<blocks, kThreads, kSmemBytes, s>>>(a, in_status);
     return cudaGetLastError();
 }
 
+namespace {
+
+// `a` from its item `first` on
+VerifyArgs items_from(VerifyArgs a, int first) {
+    const size_t i = (size_t)first;
+    a.sigs = a.sig_compressed ? (const void*)((const uint8_t*)a.sigs + 48 * i) : (const void*)((const uint64_t*)a.sigs + 12 * i);
+    a.nhms += 12 * i;
+    if (a.pk_index) {
+        a.pk_index += i;
+    } else {                    // item i has table i
+        a.pk_tables += kCoeffU64 * i;
+        if (a.pk_norm) {
+            a.pk_norm += kCoeffU64 * i;
+            a.pk_corr += 12 * i;
+        }
+        if (a.pk_identity) a.pk_identity += i;
+        a.n_keys -= first;
+    }
+    a.results += i;
+    if (a.ml_out) a.ml_out += 72 * i;
+    if (a.gt_out) a.gt_out += 72 * i;
+    if (a.sig_xy) a.sig_xy += 12 * i;
+    a.n -= first;
+    return a;
+}
+
+}  // namespace
+
+// As many lanes to an item as still give every item a place in one wave: four up
+// to 8 items a SM, two up to 16.  One launch of a block on every SM takes 3.50 ms
+// with a lane to an item, 2.77 ms with two and 2.51 ms with four (the sums shrink
+// from 2, 3, 5 and 9 products in the cyclotomic square, the line, the square and the
+// product to 1, 2, 3 and 5, or 1, 1, 2 and 3; the reductions stay).  A batch of
+// several waves whose last one would be that empty runs it as a launch of its own:
+// 4,737 items 7.0 -> 6.0 ms.
 cudaError_t launch_verify_w(const VerifyArgs& a, const uint32_t* in_status, int sms, cudaStream_t s) {
     if (a.n <= 0) return cudaSuccess;
     cudaError_t e = configure();
     if (e != cudaSuccess) return e;
-    const int need = (a.n + kV - 1) / kV;
-    int blocks = a.work_counter ? sms : need;
-    if (blocks > need) blocks = need;
-    if (blocks < 1) blocks = 1;
-    k_verify_w<<<blocks, kThreads, kSmemBytes, s>>>(a, in_status);
+    const int rest = a.n % (kV * sms);
+    const int split = rest == 0 ? 1 : rest <= 8 * sms ? 4 : rest <= 16 * sms ? 2 : 1;
+    const int full = split == 1 ? a.n : a.n - rest;   // items with a lane each
+    if (full > 0) {
+        VerifyArgs f = a;
+        f.n = full;
+        const int need = (full + kV - 1) / kV;
+        k_verify_w<1><<<f.work_counter && need > sms ? sms : need, kThreads, kSmemBytes, s>>>(f, in_status);
+        if ((e = cudaGetLastError()) != cudaSuccess || full == a.n) return e;
+    }
+    VerifyArgs t = items_from(a, full);
+    t.work_counter = nullptr;
+    const uint32_t* st = in_status ? in_status + full : nullptr;
+    const int items = kV / split, blocks = (t.n + items - 1) / items;
+    if (split == 4)
+        k_verify_w<4><<<blocks, kThreads, kSmemBytes, s>>>(t, st);
+    else
+        k_verify_w<2><<<blocks, kThreads, kSmemBytes, s>>>(t, st);
     return cudaGetLastError();
 }
 

@@ -23,6 +23,32 @@ def test_full_verify_through_programs(golden, normalised):
     T.test_full_verify_through_programs(golden, normalised)
 
 
+@pytest.mark.parametrize("lanes", [2, 4])
+def test_split_lists_hold_the_same_products(lanes):
+    """every product once, each stored sum the work of one lane from its start, and no
+    lane with more than its share by two"""
+    for name, outs, _ in G.build():
+        for c in G.pairs(outs):
+            for h in range(2 if c else 0):
+                lists = G.split_products(c, h, lanes)
+                assert sorted(p[:4] for q in lists for p in q) == sorted(p[:4] for p in c.prods[h]), name
+                want, cur = {}, []
+                for p in c.prods[h]:
+                    cur.append(p[:4])
+                    if p[4]:
+                        want[p[4][1]] = sorted(cur if p[4][0] == "sum" else cur[-1:])
+                        cur = []
+                got = {}
+                for q in lists:
+                    stores = [i for i, p in enumerate(q) if p[4]]
+                    assert len(stores) <= 1
+                    for i in stores:
+                        assert q[i][4][0] == "sum"
+                        got[q[i][4][1]] = sorted(p[:4] for p in q[:i + 1])
+                assert got == want, name
+                assert max(map(len, lists)) <= -(-len(c.prods[h]) // lanes) + 2
+
+
 def test_line_load_is_lscale():
     """the line load's descriptors name LSCALE's outputs and operands"""
     outs = dict((n, o) for n, o, _ in G.build())["LSCALE"]
