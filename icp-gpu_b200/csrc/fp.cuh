@@ -469,6 +469,25 @@ __device__ __forceinline__ fp fp_mul(const fp& a, const fp& b) {
     return r;
 }
 
+// (a b + c d) R^-1 mod p, canonical, by one reduction; a, b, c, d <= p (a row's
+// value stays below (a + c + p) 2^32, the result below 1.3p before the subtraction)
+__device__ __forceinline__ fp fp_mul2(const fp& a, const fp& b, const fp& c, const fp& d) {
+    uint32_t E[12], O[12], prev = 0;
+#pragma unroll
+    for (int i = 0; i < 12; ++i) E[i] = O[i] = 0;
+#pragma unroll
+    for (int i = 0; i < 12; ++i) {
+        mont_row_ab(E, O, prev, a.w, b.w[i]);
+        mont_row_ab(E, O, 0, c.w, d.w[i]);
+        mont_row_mp(E, O, 0);
+        prev = mont_shift(E, O);
+    }
+    fp r;
+    mont_merge(r.w, E, O, prev);
+    reduce_once(r.w);
+    return r;
+}
+
 // (t + m p) / 2^384 for the m that makes it whole: t[0..11] Montgomery-reduced
 // on its own, at most p
 __device__ __forceinline__ void mont_reduce12(uint32_t* r, const uint32_t* t) {

@@ -143,6 +143,84 @@ static __device__ __noinline__ g2j g2j_add_affine(const g2j& p, const fp2& qx, c
     return r;
 }
 
+// ---------------------------------------------------------------------------
+// Eight lanes to a key, for key sets too small to fill the chip with a lane each:
+// up to four Fp2 squares or products of one level run side by side, two lanes
+// (real, imaginary part) to each, and are handed round by shuffles.  Every lane of
+// the eight holds the point.  All 32 lanes of a warp call these together.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ fp2 oct_get(const fp& v, int j) {
+    fp2 r;
+#pragma unroll
+    for (int i = 0; i < 12; ++i) {
+        r.c0.w[i] = __shfl_sync(0xffffffffu, v.w[i], 2 * j, 8);
+        r.c1.w[i] = __shfl_sync(0xffffffffu, v.w[i], 2 * j + 1, 8);
+    }
+    return r;
+}
+__device__ __forceinline__ fp2 fp2_sel(bool c, const fp2& a, const fp2& b) {
+    return {fp_sel(c, a.c0, b.c0), fp_sel(c, a.c1, b.c1)};
+}
+// of four values the one this lane's pair works on
+__device__ __forceinline__ fp2 oct_sel(const fp2& a, const fp2& b, const fp2& c, const fp2& d) {
+    const int j = (threadIdx.x >> 1) & 3;
+    return fp2_sel(j < 2, fp2_sel(j == 0, a, b), fp2_sel(j == 2, c, d));
+}
+// this lane's part of a^2 = (a0 + a1)(a0 - a1) + 2 a0 a1 u and of a b
+__device__ __forceinline__ fp oct_sqr(const fp2& a) {
+    const bool im = threadIdx.x & 1;
+    return fp_mul(fp_add_nr(a.c0, fp_sel(im, a.c0, a.c1)), fp_sel(im, a.c1, fp_sub(a.c0, a.c1)));
+}
+__device__ __forceinline__ fp oct_mul(const fp2& a, const fp2& b) {
+    const bool im = threadIdx.x & 1;
+    return fp_mul2(a.c0, fp_sel(im, b.c1, b.c0), a.c1, fp_sel(im, b.c0, fp_neg(b.c1)));
+}
+
+// dbl-2009-l as quad_dbl (g1.cuh)
+__device__ __forceinline__ g2j oct_dbl(const g2j& p) {
+    fp s = oct_sqr(oct_sel(p.X, p.Y, fp2_add(p.Y, p.Z), p.Z));
+    const fp2 A = oct_get(s, 0), B = oct_get(s, 1);
+    g2j r;
+    r.Z = fp2_sub(fp2_sub(oct_get(s, 2), B), oct_get(s, 3));
+    const fp2 E = fp2_add(fp2_add(A, A), A);
+    s = oct_sqr(oct_sel(E, B, fp2_add(p.X, B), fp2_add(B, B)));
+    const fp2 F = oct_get(s, 0);
+    fp2 D = fp2_sub(fp2_sub(oct_get(s, 2), A), oct_get(s, 1));      // 2 X B
+    D = fp2_add(D, D);
+    r.X = fp2_sub(fp2_sub(F, D), D);
+    const fp2 C4 = oct_get(s, 3);
+    s = oct_mul(E, fp2_sub(D, r.X));                                // the same in every pair
+    r.Y = fp2_sub(oct_get(s, 0), fp2_add(C4, C4));
+    return r;
+}
+
+// p + (qx, qy), q affine (madd-2007-bl with Z3 = 2 Z1 H); *bad is set, and the
+// result of no use, when p is the identity or +-q
+static __device__ __noinline__ g2j oct_add_affine(const g2j& p, const fp2& qx, const fp2& qy, bool* bad) {
+    fp s = oct_mul(oct_sel(p.Z, qy, p.Z, qy), p.Z);                 // Z^2, qy Z
+    const fp2 ZZ = oct_get(s, 0);
+    s = oct_mul(oct_sel(qx, oct_get(s, 1), qx, qx), ZZ);            // U2, S2
+    const fp2 H = fp2_sub(oct_get(s, 0), p.X);
+    fp2 rr = fp2_sub(oct_get(s, 1), p.Y);
+    rr = fp2_add(rr, rr);
+    if (fp2_is_zero(p.Z) || fp2_is_zero(H)) *bad = true;
+    s = oct_mul(oct_sel(H, rr, H, H), oct_sel(H, rr, p.Z, H));      // H^2, rr^2, H Z
+    fp2 I = oct_get(s, 0);
+    I = fp2_add(I, I);
+    I = fp2_add(I, I);
+    const fp2 rr2 = oct_get(s, 1);
+    g2j r;
+    r.Z = oct_get(s, 2);
+    r.Z = fp2_add(r.Z, r.Z);
+    s = oct_mul(oct_sel(H, p.X, H, H), I);                          // J, V
+    const fp2 J = oct_get(s, 0), V = oct_get(s, 1);
+    r.X = fp2_sub(fp2_sub(rr2, J), fp2_add(V, V));
+    s = oct_mul(oct_sel(rr, p.Y, rr, rr), oct_sel(fp2_sub(V, r.X), J, J, J));
+    const fp2 YJ = oct_get(s, 1);
+    r.Y = fp2_sub(oct_get(s, 0), fp2_add(YJ, YJ));
+    return r;
+}
+
 // psi(P) == [x] P for an affine point P on the twist (not the identity), x the
 // BLS parameter -0xd201000000010000.  psi(x, y) = (conj(x) cx, conj(y) cy)
 // with cx = (1 + u)^(-(p-1)/3), cy = (1 + u)^(-(p-1)/2) is the untwist-
@@ -150,6 +228,7 @@ static __device__ __noinline__ g2j g2j_add_affine(const g2j& p, const fp2& qx, c
 // (Scott, eprint 2021/1130 section 4; proof El Housni, Guillevic and
 // Piellard, eprint 2022/352).  63 doublings and 5 additions, against 254 and
 // 133 for [r] P == O.
+static __device__ __noinline__ bool g2_is_psi(const fp2& x, const fp2& y, const g2j& acc);
 static __device__ __noinline__ bool g2_in_subgroup(const fp2& x, const fp2& y) {
     const uint64_t xabs = 0xd201000000010000ULL;
     g2j acc = {x, y, fp2_one()};
@@ -157,6 +236,23 @@ static __device__ __noinline__ bool g2_in_subgroup(const fp2& x, const fp2& y) {
         acc = g2j_dbl(acc);
         if ((xabs >> i) & 1) acc = g2j_add_affine(acc, x, y);
     }
+    return g2_is_psi(x, y, acc);
+}
+// the same with eight lanes to the point.  No k P with 1 < k <= |x| is the identity
+// or +-P for a P of order r, so a point that meets an exceptional addition is outside.
+static __device__ __noinline__ bool oct_in_subgroup(const fp2& x, const fp2& y) {
+    const uint64_t xabs = 0xd201000000010000ULL;
+    g2j acc = {x, y, fp2_one()};
+    bool bad = false;
+#pragma unroll 1
+    for (int i = 62; i >= 0; --i) {
+        acc = oct_dbl(acc);
+        if ((xabs >> i) & 1) acc = oct_add_affine(acc, x, y, &bad);
+    }
+    return !bad && g2_is_psi(x, y, acc);
+}
+// psi(x, y) == -acc for acc = [|x|] P
+static __device__ __noinline__ bool g2_is_psi(const fp2& x, const fp2& y, const g2j& acc) {
     if (fp2_is_zero(acc.Z)) return false;
     // Montgomery forms: cx = (0, cx1), cy = (cy0, cy1)
     const uint64_t cx1[6] = {0x890dc9e4867545c3ULL, 0x2af322533285a5d5ULL, 0x50880866309b7e2cULL,
@@ -189,7 +285,7 @@ __device__ __forceinline__ fp fp_from_be48(const uint8_t* in, bool mask_flags) {
 
 // Decode one 96-byte key.  On success writes Montgomery (x, y); the identity
 // is reported by *identity (and x = y = 0).  Returns a status code.
-__device__ __forceinline__ int32_t g2_decode(const uint8_t* in, fp2& x, fp2& y, bool& identity) {
+__device__ __forceinline__ int32_t g2_decode(const uint8_t* in, fp2& x, fp2& y, bool& identity, bool check_subgroup) {
     identity = false;
     x = fp2_zero();
     y = fp2_zero();
@@ -210,7 +306,7 @@ __device__ __forceinline__ int32_t g2_decode(const uint8_t* in, fp2& x, fp2& y, 
     fp2 yy = fp2_sqrt(y2, &ok);
     if (!ok) return ST_NOT_ON_CURVE;
     if (fp2_lex_largest(yy) != sort) yy = fp2_neg(yy);
-    if (!g2_in_subgroup(xm, yy)) return ST_NOT_IN_SUBGROUP;
+    if (check_subgroup && !g2_in_subgroup(xm, yy)) return ST_NOT_IN_SUBGROUP;
     x = xm;
     y = yy;
     return ST_OK;

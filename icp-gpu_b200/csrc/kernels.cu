@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(64) k_g2_decompress(const uint8_t* in, int n, 
     if (i >= n) return;
     fp2 x, y;
     bool id;
-    int32_t st = g2_decode(in + 96 * (size_t)i, x, y, id);
+    int32_t st = g2_decode(in + 96 * (size_t)i, x, y, id, true);
     status[i] = st;
     uint64_t* qi = q + 24 * (size_t)i;
     store_fp2(qi, x);
@@ -171,6 +171,42 @@ __global__ void __launch_bounds__(64) k_g2_prepare(const uint64_t* q, int n, uin
     fp2 qx = {fp_load_u64(qi), fp_load_u64(qi + 6)};
     fp2 qy = {fp_load_u64(qi + 12), fp_load_u64(qi + 18)};
     g2_prepare(qx, qy, out + BLS_COEFF_U64 * (size_t)i);
+}
+
+// Both for key sets too small to fill the chip: eight lanes to a key (g2.cuh,
+// g2prep.cuh), four keys a warp.  Bound by one key's chain
+// (two powers and 63 doublings; 63 doublings and 5 additions with their lines).
+constexpr int kOctThreads = 32;
+__global__ void __launch_bounds__(kOctThreads) k_g2_decompress_oct(const uint8_t* in, int n, uint64_t* q, int32_t* status,
+                                                                   uint8_t* identity) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, l = t & 7;
+    const int i = (t >> 3) < n ? (t >> 3) : n - 1;   // past the end: the last key again, the warp stays together
+    fp2 x, y;
+    bool id;
+    int32_t st = g2_decode(in + 96 * (size_t)i, x, y, id, false);
+    __syncwarp();
+    const bool test = st == ST_OK && !id;
+    const fp2 one = fp2_one();                       // any point will do where there is none to test
+    const bool ok = oct_in_subgroup(fp2_sel(test, x, one), fp2_sel(test, y, one));
+    if (test && !ok) {
+        st = ST_NOT_IN_SUBGROUP;
+        x = y = fp2_zero();
+    }
+    if ((t >> 3) >= n) return;
+    if (l < 4) fp_store_u64(q + 24 * (size_t)i + 6 * l, fp_sel(l < 2, fp_sel(l == 0, x.c0, x.c1), fp_sel(l == 2, y.c0, y.c1)));
+    if (l == 0) {
+        status[i] = st;
+        if (identity) identity[i] = (st == ST_OK && id) ? 1 : 0;
+    }
+}
+
+__global__ void __launch_bounds__(kOctThreads) k_g2_prepare_oct(const uint64_t* q, int n, uint64_t* out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool live = (t >> 3) < n;
+    const int i = live ? (t >> 3) : n - 1;
+    const uint64_t* qi = q + 24 * (size_t)i;
+    const fp2 qx = {fp_load_u64(qi), fp_load_u64(qi + 6)}, qy = {fp_load_u64(qi + 12), fp_load_u64(qi + 18)};
+    oct_prepare(qx, qy, out + BLS_COEFF_U64 * (size_t)i, live);
 }
 
 // Small key sets: one line table per block, one row per thread, so a table's
@@ -303,8 +339,9 @@ __global__ void __launch_bounds__(64) k_lines_normalize_table(const uint64_t* ra
 // A key set of at most kRowsMaxTables tables takes the row-parallel form (low
 // latency: one block per table); a larger one the table-per-thread form
 // (least work: the whole set in one wave, where the row form would square each
-// row's c2 separately and take many waves).
-constexpr int kRowsMaxTables = 2048;
+// row's c2 separately and take many waves).  With the line tables themselves: 2,368
+// keys 2.11 against 2.53 ms, 4,736 keys 3.80 against 2.80 ms.
+constexpr int kRowsMaxTables = 2960;
 
 cudaError_t launch_lines_normalize(const uint64_t* raw, int n, uint64_t* norm, uint64_t* corr, uint8_t* bad,
                                    cudaStream_t s) {
@@ -365,16 +402,28 @@ cudaError_t launch_g1_subgroup_sms(const uint64_t* xy, const int32_t* status, in
     return cudaGetLastError();
 }
 
+// From host buffers, eight lanes against one: bls_g2_decompress_status of 500 keys
+// 1.35 and 2.30 ms, 2,368 keys (a warp on every scheduler) 1.43 and 2.37 ms, 4,736
+// keys 2.11 and 2.46 ms, 9,472 keys 4.09 and 2.61 ms; bls_pk_register_affine_batch of
+// 500 keys 0.96 and 2.59 ms, 4,736 keys 2.80 and 4.20 ms, 9,472 keys 3.71 and 4.30 ms.
+constexpr int kOctMaxKeys = 4736;
+
 cudaError_t launch_g2_decompress(const uint8_t* in, int n, uint64_t* q, int32_t* status, uint8_t* identity,
                                  cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    k_g2_decompress<<<(n + 63) / 64, 64, 0, s>>>(in, n, q, status, identity);
+    if (n <= kOctMaxKeys)
+        k_g2_decompress_oct<<<(8 * n + kOctThreads - 1) / kOctThreads, kOctThreads, 0, s>>>(in, n, q, status, identity);
+    else
+        k_g2_decompress<<<(n + 63) / 64, 64, 0, s>>>(in, n, q, status, identity);
     return cudaGetLastError();
 }
 
 cudaError_t launch_g2_prepare(const uint64_t* q, int n, uint64_t* out, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    k_g2_prepare<<<(n + 63) / 64, 64, 0, s>>>(q, n, out);
+    if (n <= kOctMaxKeys)
+        k_g2_prepare_oct<<<(8 * n + kOctThreads - 1) / kOctThreads, kOctThreads, 0, s>>>(q, n, out);
+    else
+        k_g2_prepare<<<(n + 63) / 64, 64, 0, s>>>(q, n, out);
     return cudaGetLastError();
 }
 
