@@ -60,13 +60,14 @@ __device__ __forceinline__ bool fp_lex_largest(const fp& a) {
 struct g1j { fp X, Y, Z; };
 
 // The Jacobian routines run one thread per point, a few warps per scheduler:
-// their products are the out-of-line multiply of fp.cuh.
+// their products are the out-of-line multiply of fp.cuh, and a sum that is squared
+// (below 3p) or multiplied (below 8p) next is left unreduced.
 // dbl-2009-l (a = 0)
 static __device__ __noinline__ g1j g1j_dbl(const g1j& p) {
     fp A = fp_sqr_ool(p.X), B = fp_sqr_ool(p.Y), C = fp_sqr_ool(B);
-    fp D = fp_sub(fp_sub(fp_sqr_ool(fp_add(p.X, B)), A), C);
+    fp D = fp_sub(fp_sub(fp_sqr_ool(fp_add_nr(p.X, B)), A), C);
     D = fp_add(D, D);
-    fp E = fp_add(fp_add(A, A), A);
+    fp E = fp_add_nr(fp_add_nr(A, A), A);
     fp F = fp_sqr_ool(E);
     g1j r;
     r.X = fp_sub(F, fp_add(D, D));
@@ -74,7 +75,7 @@ static __device__ __noinline__ g1j g1j_dbl(const g1j& p) {
     C8 = fp_add(C8, C8);
     C8 = fp_add(C8, C8);
     r.Y = fp_sub(fp_mul_ool(E, fp_sub(D, r.X)), C8);
-    r.Z = fp_mul_ool(fp_add(p.Y, p.Y), p.Z);
+    r.Z = fp_mul_ool(fp_add_nr(p.Y, p.Y), p.Z);
     return r;
 }
 
@@ -90,17 +91,17 @@ static __device__ __noinline__ g1j g1j_add_affine(const g1j& p, const fp& qx, co
         if (fp_is_zero(rr)) return g1j_dbl(p);
         return {fp_one(), fp_one(), fp_zero()};
     }
-    rr = fp_add(rr, rr);
+    rr = fp_add_nr(rr, rr);
     fp HH = fp_sqr_ool(H);
-    fp I = fp_add(HH, HH);
-    I = fp_add(I, I);
+    fp I = fp_add_nr(HH, HH);
+    I = fp_add_nr(I, I);
     fp J = fp_mul_ool(H, I);
     fp V = fp_mul_ool(p.X, I);
     g1j r;
     r.X = fp_sub(fp_sub(fp_sqr_ool(rr), J), fp_add(V, V));
     fp YJ = fp_mul_ool(p.Y, J);
     r.Y = fp_sub(fp_mul_ool(rr, fp_sub(V, r.X)), fp_add(YJ, YJ));
-    r.Z = fp_sub(fp_sub(fp_sqr_ool(fp_add(p.Z, H)), Z1Z1), HH);
+    r.Z = fp_sub(fp_sub(fp_sqr_ool(fp_add_nr(p.Z, H)), Z1Z1), HH);
     return r;
 }
 
@@ -117,16 +118,16 @@ static __device__ __noinline__ g1j g1j_add(const g1j& p, const g1j& q) {
         if (fp_is_zero(rr)) return g1j_dbl(p);
         return {fp_one(), fp_one(), fp_zero()};
     }
-    fp I = fp_add(H, H);
+    fp I = fp_add_nr(H, H);
     I = fp_sqr_ool(I);
     const fp J = fp_mul_ool(H, I);
-    rr = fp_add(rr, rr);
+    rr = fp_add_nr(rr, rr);
     const fp V = fp_mul_ool(U1, I);
     g1j r;
     r.X = fp_sub(fp_sub(fp_sqr_ool(rr), J), fp_add(V, V));
     const fp SJ = fp_mul_ool(S1, J);
     r.Y = fp_sub(fp_mul_ool(rr, fp_sub(V, r.X)), fp_add(SJ, SJ));
-    r.Z = fp_mul_ool(fp_sub(fp_sub(fp_sqr_ool(fp_add(p.Z, q.Z)), Z1Z1), Z2Z2), H);
+    r.Z = fp_mul_ool(fp_sub(fp_sub(fp_sqr_ool(fp_add_nr(p.Z, q.Z)), Z1Z1), Z2Z2), H);
     return r;
 }
 

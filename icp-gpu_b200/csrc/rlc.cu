@@ -86,10 +86,13 @@ static __device__ __noinline__ bool g1_point_ok(const fp& x, const fp& y) {
     return g1_in_subgroup(x, y);
 }
 
-// A block of four warps takes 32 items; warp w has role w for all of them
+// A block of four warps takes 32 items; each warp has one role for all of them
 // (0: [r] sig, 1: [r] nhm, 2: sig checks, 3: nhm checks), so a warp never
-// splits between the scalar multiplication and the checks.
-__global__ void __launch_bounds__(128) k_rlc_scale(const uint64_t* sig_xy, const int32_t* status,
+// splits between the scalar multiplication and the checks.  Bound by the multiply
+// pipe and its carries; four blocks an SM (128 registers) instead of two: 16,384
+// items 2.89 -> 2.37 ms.  (The roles moved on by one warp from block to block,
+// which evens the schedulers out, 2.63 ms.)
+__global__ void __launch_bounds__(128, 4) k_rlc_scale(const uint64_t* sig_xy, const int32_t* status,
                                                    const uint64_t* nhms, const uint64_t* r, int n, int check_sig,
                                                    uint32_t* pts, uint8_t* bad, int* counters) {
     const int role = threadIdx.x >> 5;
@@ -114,35 +117,29 @@ __global__ void __launch_bounds__(128) k_rlc_scale(const uint64_t* sig_xy, const
 
 // tile t: items order[tile[3t] .. tile[3t + 1]) (one key); partials: signature
 // sum then key sum, 72 words per tile
-__global__ void __launch_bounds__(kTileThreads) k_rlc_tiles(const uint32_t* pts, const int32_t* order,
-                                                            const int32_t* tiles, uint32_t* partials) {
-    __shared__ uint32_t sm[kTileThreads][36];
+__global__ void __launch_bounds__(2 * kTileThreads) k_rlc_tiles(const uint32_t* pts, const int32_t* order,
+                                                                const int32_t* tiles, uint32_t* partials) {
+    __shared__ uint32_t sm[2 * kTileThreads][36];
     const int a = tiles[3 * blockIdx.x], b = tiles[3 * blockIdx.x + 1];
-    g1j acc[2];
-    for (int s = 0; s < 2; ++s) {
-        acc[s] = g1j_identity();
-        for (int k = a + threadIdx.x; k < b; k += kTileThreads)
-            acc[s] = g1j_add(acc[s], load_j(pts + 72 * (size_t)order[k] + 36 * s));
-        store_j(sm[threadIdx.x], acc[s]);
-        __syncthreads();
-        for (int w = kTileThreads / 2; w > 0; w >>= 1) {
-            if ((int)threadIdx.x < w) {
-                acc[s] = g1j_add(acc[s], load_j(sm[threadIdx.x + w]));
-                store_j(sm[threadIdx.x], acc[s]);
-            }
-            __syncthreads();
+    const int s = threadIdx.x / kTileThreads, t = threadIdx.x % kTileThreads;   // the two sums side by side
+    g1j acc = g1j_identity();
+    for (int k = a + t; k < b; k += kTileThreads) acc = g1j_add(acc, load_j(pts + 72 * (size_t)order[k] + 36 * s));
+    store_j(sm[threadIdx.x], acc);
+    __syncthreads();
+    for (int w = kTileThreads / 2; w > 0; w >>= 1) {
+        if (t < w) {
+            acc = g1j_add(acc, load_j(sm[threadIdx.x + w]));
+            store_j(sm[threadIdx.x], acc);
         }
-        if (threadIdx.x == 0) store_j(partials + 72 * (size_t)blockIdx.x + 36 * s, acc[s]);
         __syncthreads();
     }
+    if (t == 0) store_j(partials + 72 * (size_t)blockIdx.x + 36 * s, acc);
 }
 
 __device__ __forceinline__ void store_affine(uint64_t* d, const g1j& p) {
     fp x = fp_zero(), y = fp_one();   // the identity: x = 0, y = R mod p
     if (!fp_is_zero(p.Z)) {
-        const uint64_t pm2[6] = {0xb9feffffffffaaa9ULL, 0x1eabfffeb153ffffULL, 0x6730d2a0f6b0f624ULL,
-                                 0x64774b84f38512bfULL, 0x4b1ba7b6434bacd7ULL, 0x1a0111ea397fe69aULL};  // p - 2
-        const fp zi = fp_pow_u64(p.Z, pm2, 381), zi2 = fp_sqr(zi);
+        const fp zi = fp_inv(p.Z), zi2 = fp_sqr(zi);
         x = fp_mul(p.X, zi2);
         y = fp_mul(p.Y, fp_mul(zi2, zi));
     }
@@ -169,17 +166,42 @@ __global__ void __launch_bounds__(256) k_rlc_final(const uint32_t* partials, int
         g1j h = g1j_identity();
         for (int t = key_tile[k]; t < key_tile[k + 1]; ++t) h = g1j_add(h, load_j(partials + 72 * (size_t)t + 36));
         store_affine(out_nhms + 12 * (size_t)k, h);
-        if (k == 0) store_affine(out_sigs, s);
-        else store_affine(out_sigs + 12 * (size_t)k, g1j_identity());
+        if (k > 0) store_affine(out_sigs + 12 * (size_t)k, g1j_identity());
     }
+    // the signature sum's affine form on the last warp, beside the first keys'
+    if (threadIdx.x == 224) store_affine(out_sigs, load_j(sm[0]));
 }
 
-// product of n Gt values (in place), counters[0] = 1 when it is one
-__global__ void __launch_bounds__(128) k_gt_product(uint64_t* gt, int n, int* counters) {
+// product of n Gt values (in place), counters[0] = 1 when it is one: a tree, six
+// threads to a product, each the sum of the six Fp2 products of one coefficient in
+// the basis 1, w, .., w^5 (w^6 = xi; tower position t holds the power kW[t]).  A
+// lone thread's 54 products a level made the tree of 40 values 0.44 ms, this 0.14.
+constexpr int kGtThreads = 6 * 64;
+__global__ void __launch_bounds__(kGtThreads) k_gt_product(uint64_t* gt, int n, int* counters) {
+    constexpr int kW[6] = {0, 2, 4, 1, 3, 5}, kT[6] = {0, 3, 1, 4, 2, 5};
+    const int t = threadIdx.x % 6, k = kW[t];
     for (int w = 1; w < n; w <<= 1) {
-        for (int i = 2 * w * threadIdx.x; i + w < n; i += 2 * w * blockDim.x)
-            fp12_store_u64(gt + 72 * (size_t)i, fp12_mul(fp12_load_u64(gt + 72 * (size_t)i),
-                                                         fp12_load_u64(gt + 72 * (size_t)(i + w))));
+        for (int base = 0; base + w < n; base += 2 * w * (kGtThreads / 6)) {
+            const int i = base + 2 * w * (threadIdx.x / 6);
+            const bool live = i + w < n;
+            fp2 sum = fp2_zero(), over = fp2_zero();
+            if (live) {
+                const uint64_t *a = gt + 72 * (size_t)i, *b = gt + 72 * (size_t)(i + w);
+#pragma unroll 1
+                for (int j = 0; j < 6; ++j) {
+                    const int o = (k - j + 6) % 6;
+                    const fp2 v = fp2_mul(load_fp2(a + 12 * kT[j]), load_fp2(b + 12 * kT[o]));
+                    if (j > k) over = fp2_add(over, v);
+                    else sum = fp2_add(sum, v);
+                }
+                sum = fp2_add(sum, fp2_mul_nr(over));
+            }
+            __syncthreads();                         // every coefficient read before one is written
+            if (live) {
+                fp_store_u64(gt + 72 * (size_t)i + 12 * t, sum.c0);
+                fp_store_u64(gt + 72 * (size_t)i + 12 * t + 6, sum.c1);
+            }
+        }
         __syncthreads();
     }
     if (threadIdx.x == 0) counters[0] = fp12_is_one(fp12_load_u64(gt)) ? 1 : 0;
@@ -191,14 +213,14 @@ cudaError_t launch_rlc(const RlcArgs& a, cudaStream_t s) {
     if (a.n <= 0 || a.ntiles <= 0 || a.nkeys <= 0) return cudaErrorInvalidValue;
     k_rlc_scale<<<(unsigned)((a.n + 31) / 32), 128, 0, s>>>(a.sig_xy, a.status, a.nhms, a.r, a.n, a.check_sig,
                                                                  a.pts, a.bad, a.counters);
-    k_rlc_tiles<<<a.ntiles, kTileThreads, 0, s>>>(a.pts, a.order, a.tiles, a.partials);
+    k_rlc_tiles<<<a.ntiles, 2 * kTileThreads, 0, s>>>(a.pts, a.order, a.tiles, a.partials);
     k_rlc_final<<<1, 256, 0, s>>>(a.partials, a.ntiles, a.key_tile, a.nkeys, a.agg_sigs, a.agg_nhms);
     return cudaGetLastError();
 }
 
 cudaError_t launch_gt_product(uint64_t* gt, int n, int* counters, cudaStream_t s) {
     if (n <= 0) return cudaErrorInvalidValue;
-    k_gt_product<<<1, 128, 0, s>>>(gt, n, counters);
+    k_gt_product<<<1, kGtThreads, 0, s>>>(gt, n, counters);
     return cudaGetLastError();
 }
 
