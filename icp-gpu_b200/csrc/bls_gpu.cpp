@@ -419,8 +419,10 @@ int run_verify(bls_ctx* c, bls::VerifyArgs a) {
     return BLS_OK;
 }
 
-// grow every buffer a verify of n staged items needs (nothing allocates after)
-int prepare(bls_ctx* c, size_t n, int fmt, bool want_ml, bool want_gt) {
+// grow every buffer a verify of n items needs (nothing allocates after); staged:
+// the inputs go through pinned staging (pinned buffers cost milliseconds to
+// allocate, and a call that copies straight from its caller's needs none)
+int prepare(bls_ctx* c, size_t n, int fmt, bool want_ml, bool want_gt, bool staged) {
     size_t sig_bytes = n * (fmt == BLS_SIG_COMPRESSED ? 48 : 96);
     int rc;
     if ((rc = c->grow(c->d_sigs, sig_bytes)) || (rc = c->grow(c->d_nhms, n * 96)) ||
@@ -429,10 +431,10 @@ int prepare(bls_ctx* c, size_t n, int fmt, bool want_ml, bool want_gt) {
     if (fmt == BLS_SIG_COMPRESSED && ((rc = c->grow(c->d_xy, n * 96)) || (rc = c->grow(c->d_st, n * 4)))) return rc;
     if (want_ml && (rc = c->grow(c->d_ml, n * 576))) return rc;
     if (want_gt && (rc = c->grow(c->d_gt, n * 576))) return rc;
-    if ((rc = c->grow(c->h_sigs, sig_bytes)) || (rc = c->grow(c->h_nhms, n * 96)) ||
-        (rc = c->grow(c->h_pkidx, n * 4)) || (rc = c->grow(c->h_res, n * 4)))
+    if (staged && ((rc = c->grow(c->h_sigs, sig_bytes)) || (rc = c->grow(c->h_nhms, n * 96)) ||
+                   (rc = c->grow(c->h_pkidx, n * 4))))
         return rc;
-    return BLS_OK;
+    return c->grow(c->h_res, n * 4);
 }
 
 // enqueue: staged inputs -> device, verify, results -> h_res (no synchronise);
@@ -846,7 +848,7 @@ int bls_verify_batch(bls_ctx* ctx, const bls_batch* b, int32_t* results) {
     CK(cudaSetDevice(ctx->cfg.device));
     size_t n = (size_t)b->n;
     size_t sig_bytes = n * (b->sig_format == BLS_SIG_COMPRESSED ? 48 : 96);
-    if ((rc = prepare(ctx, n, b->sig_format, b->miller_out != nullptr, b->gt_out != nullptr))) return rc;
+    if ((rc = prepare(ctx, n, b->sig_format, b->miller_out != nullptr, b->gt_out != nullptr, false))) return rc;
     // the caller's buffers straight to the device (the call is synchronous, so
     // they outlive the copies): the driver pipelines a pageable copy through
     // its own staging, where a copy into pinned staging first would serialise
@@ -886,7 +888,7 @@ int bls_verify_requests(bls_ctx* ctx, const bls_request* reqs, int nreq, int fmt
         for (int r = 0; r < nreq; ++r) {
             size_t n = (size_t)reqs[r].n;
             if (!n) continue;
-            if ((rc = prepare(ctx, n, fmt, false, false))) return rc;
+            if ((rc = prepare(ctx, n, fmt, false, false, true))) return rc;
             memcpy(ctx->h_sigs.p, reqs[r].sigs, n * sb);
             memcpy(ctx->h_nhms.p, reqs[r].neg_hms, n * 96);
             memcpy(ctx->h_pkidx.p, reqs[r].pk_ids, n * 4);
@@ -896,7 +898,7 @@ int bls_verify_requests(bls_ctx* ctx, const bls_request* reqs, int nreq, int fmt
         }
         return BLS_OK;
     }
-    if ((rc = prepare(ctx, total, fmt, false, false))) return rc;
+    if ((rc = prepare(ctx, total, fmt, false, false, true))) return rc;
     // every request into the pinned staging at its offset, on the host's cores
     std::vector<size_t> first((size_t)nreq + 1, 0);
     for (int r = 0; r < nreq; ++r) first[r + 1] = first[r] + (size_t)reqs[r].n;
@@ -1142,17 +1144,14 @@ int bls_verify_batch_rlc(bls_ctx* ctx, const bls_batch* b, const uint64_t* scala
                  o_til = o_ord + al(n * 4), o_kt = o_til + al(tiles.size() * 4),
                  o_key = o_kt + al(key_tile.size() * 4), o_bad = o_key + al((size_t)nkeys * 4),
                  o_res = o_bad + al(n * 2), o_cnt = o_res + al((size_t)nkeys * 4), total = o_cnt + 256;
-    if ((rc = prepare(ctx, n, fmt, false, false)) || (rc = ctx->grow(ctx->d_rlc, total)) ||
+    if ((rc = prepare(ctx, n, fmt, false, false, false)) || (rc = ctx->grow(ctx->d_rlc, total)) ||
         (rc = ctx->grow(ctx->d_gt, (size_t)nkeys * 576)))
         return rc;
     uint8_t* base = (uint8_t*)ctx->d_rlc.p;
     const size_t sig_bytes = n * (fmt == BLS_SIG_COMPRESSED ? 48 : 96);
-    memcpy(ctx->h_sigs.p, b->sigs, sig_bytes);
-    memcpy(ctx->h_nhms.p, b->neg_hms, n * 96);
-    memcpy(ctx->h_pkidx.p, b->pk_ids, n * 4);
     cudaStream_t st = ctx->stream;
-    CK(cudaMemcpyAsync(ctx->d_sigs.p, ctx->h_sigs.p, sig_bytes, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(ctx->d_nhms.p, ctx->h_nhms.p, n * 96, cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(ctx->d_sigs.p, b->sigs, sig_bytes, cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(ctx->d_nhms.p, b->neg_hms, n * 96, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(base + o_r, r.data(), n * 8, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(base + o_ord, order.data(), n * 4, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(base + o_til, tiles.data(), tiles.size() * 4, cudaMemcpyHostToDevice, st));
@@ -1215,8 +1214,9 @@ int bls_verify_batch_rlc(bls_ctx* ctx, const bls_batch* b, const uint64_t* scala
             for (size_t i = 0; i < n; ++i) results[i] = BLS_ACCEPT;
         }
     } else {
-        // the per-item path on the staged inputs
-        if ((rc = enqueue(ctx, n, fmt, false, false, false))) return rc;
+        // the per-item path on the inputs already there
+        CK(cudaMemcpyAsync(ctx->d_pkidx.p, b->pk_ids, n * 4, cudaMemcpyHostToDevice, st));
+        if ((rc = enqueue(ctx, n, fmt, false, false, false, false, true))) return rc;
         CK(cudaStreamSynchronize(st));
         memcpy(results, ctx->h_res.p, n * 4);
     }
@@ -1250,7 +1250,7 @@ int bls_verify_messages(bls_ctx* ctx, int fmt, const void* sigs, const uint8_t* 
     if ((rc = check_ids(ctx, pk_ids, n))) return rc;
     CK(cudaSetDevice(ctx->cfg.device));
     const size_t k = (size_t)n;
-    if ((rc = prepare(ctx, k, fmt, false, false))) return rc;
+    if ((rc = prepare(ctx, k, fmt, false, false, false))) return rc;
     CK(cudaMemcpyAsync(ctx->d_sigs.p, sigs, k * (fmt == BLS_SIG_COMPRESSED ? 48 : 96), cudaMemcpyHostToDevice,
                        ctx->stream));
     CK(cudaMemcpyAsync(ctx->d_pkidx.p, pk_ids, k * 4, cudaMemcpyHostToDevice, ctx->stream));
