@@ -390,7 +390,21 @@ __device__ __forceinline__ void run(int pid, const Sm& s, int k, int half, const
         }
         store_fp(s, slot_addr(bs, (hdr >> 8) & 0x7fu), half, o);
     }
-    __syncthreads();
+}
+
+// The meeting after a program, before the op `next` (a code): the whole block's,
+// but for two cases in which fewer warps, or none, have anything to wait for.
+// From one cyclotomic square to the next (groups A and D change places) the
+// values fall into two sets that do not read each other: coefficients 0 and 4, and
+// the rest.  And a line load after a square reads no Fp12 value and writes line
+// slots that were last read before the square.
+__device__ __forceinline__ void meet(uint32_t code, uint32_t next, int k) {
+    if (code == (uint32_t)f2::P_CYCSQR && next == (uint32_t)f2::P_CYCSQR) {
+        if (k == 0 || k == 4) asm volatile("bar.sync 7, 128;" ::: "memory");
+        else asm volatile("bar.sync 8, 256;" ::: "memory");
+    } else if (!(code == (uint32_t)f2::P_SQR && next == f2::kOpLoadLines)) {
+        __syncthreads();
+    }
 }
 
 __device__ __forceinline__ uint32_t grp(int g) { return kKSlots + 6 * g; }
@@ -646,6 +660,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_verify_w(VerifyArgs a, const ui
             }
             if (code < (uint32_t)f2::kNumPrograms || code == f2::kOpLoadLines) {
                 run<kSplit>(pid, s, k, half, bs, line);
+                meet(code, st + 1 < seq_len ? f2::kSeq[norm][st + 1] & 31u : 0u, k);
             } else if (code == f2::kOpLoadCorr) {
                 // the generator's and the key's Miller correction factors into the c2 slots
                 if (k < 2) {
