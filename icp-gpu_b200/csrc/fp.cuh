@@ -704,7 +704,6 @@ __device__ __forceinline__ fp fp_sub(const fp& a, const fp& b) {
 }
 
 __device__ __forceinline__ fp fp_neg(const fp& a) { return fp_sub(fp_zero(), a); }
-__device__ __forceinline__ fp fp_dbl(const fp& a) { return fp_add(a, a); }
 
 // ---------------------------------------------------------------------------
 // conversions
@@ -735,16 +734,6 @@ __device__ __forceinline__ fp fp_to_mont(const fp& a) { return fp_mul(a, fp_rr()
 __device__ __forceinline__ bool fp_raw_geq_p(const fp& a) {
     uint32_t d[12];
     return sub_p(d, a.w) == 0;
-}
-
-// a^e for a fixed exponent given as 6 little-endian u64 words (right to left)
-__device__ __forceinline__ fp fp_pow_u64(const fp& a, const uint64_t* e, int nbits) {
-    fp r = fp_one(), base = a;
-    for (int i = 0; i < nbits; ++i) {
-        if ((e[i >> 6] >> (i & 63)) & 1) r = fp_mul(r, base);
-        base = fp_sqr(base);
-    }
-    return r;
 }
 
 // An out-of-line Montgomery multiply and square, and a power over them, for

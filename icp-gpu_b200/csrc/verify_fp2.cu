@@ -552,9 +552,9 @@ __global__ void __launch_bounds__(kThreads, 6) k_verify_fp2(VerifyArgs a, const 
 size_t smem_bytes() { return (size_t)(kSlotArea + kXchArea + kFlagArea + 16 * kKpCount) * 4; }
 
 // The carry-chain ceiling the verify kernel is measured against: every thread
-// runs `iters` schoolbook 12 x 12-limb products (prod24: 144 mul.lo + 144
-// mul.hi chained through the carry flag, 288 IMAD-pipe instructions) and adds each into a
-// 26-limb accumulator, with the verify kernel's block shape and occupancy and
+// runs `iters` schoolbook 12 x 12-limb products (prod24: 144 pairs of mul.lo and
+// mul.hi chained through the carry flag, counted as 288 multiplies) and adds each
+// into a 26-limb accumulator, with the verify kernel's block shape and occupancy and
 // no loads, barriers or reductions; one operand changes every iteration so
 // no product can be hoisted.
 __global__ void __launch_bounds__(kThreads, 6) k_imad_chain(int iters, uint32_t* out) {
