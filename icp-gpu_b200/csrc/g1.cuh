@@ -275,8 +275,10 @@ static __device__ __noinline__ bool quad_in_subgroup(const fp& x, const fp& y) {
     s = fp_mul_ool(Z2, fp_sel(l == 0, acc.Z, quad_get(s, 1)));                              // Z^3, beta x Z^2
     const fp Z3 = quad_get(s, 0), bx = quad_get(s, 1);
     const bool ok = fp_eq(acc.X, bx) && fp_is_zero(fp_add(acc.Y, fp_mul_ool(y, Z3)));
-    // a point of small order met an exceptional addition: one lane, all cases handled
-    return bad ? g1_in_subgroup(x, y) : (ok && !fp_is_zero(acc.Z));
+    // a point of small order met an exceptional addition: one lane, all cases handled.
+    // x = 0, the identity's encoding among them, is a point of order 3, outside without
+    // that second chain (448 encodings with an identity: 1.60 -> 0.59 ms).
+    return bad ? (!fp_is_zero(x) && g1_in_subgroup(x, y)) : (ok && !fp_is_zero(acc.Z));
 }
 
 // x of a 48-byte encoding as an integer, the flag bits off
