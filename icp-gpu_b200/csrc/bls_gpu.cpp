@@ -395,8 +395,9 @@ int default_ctx(bls_ctx** out) {
 // One verify launch on the context stream.  lanes_per_pairing 1 runs the
 // thread-per-verification kernel (which decodes compressed signatures itself);
 // otherwise compressed signatures are first decoded into scratch buffers by
-// one thread per point, then the lane-parallel kernel verifies.
-int run_verify(bls_ctx* c, bls::VerifyArgs a) {
+// launch_g1_decompress, then the lane-parallel kernel verifies; decoded: d_xy and
+// d_st already hold them.
+int run_verify(bls_ctx* c, bls::VerifyArgs a, bool decoded = false) {
     if (c->cfg.lanes_per_pairing == 1) {
         a.work_counter = nullptr;
         CK(bls::launch_verify(a, c->stream));
@@ -408,8 +409,9 @@ int run_verify(bls_ctx* c, bls::VerifyArgs a) {
         if ((c->d_xy.cap < (size_t)a.n * 96 || c->d_st.cap < (size_t)a.n * 4) &&
             ((rc = c->grow(c->d_xy, (size_t)a.n * 96)) || (rc = c->grow(c->d_st, (size_t)a.n * 4))))
             return rc;
-        CK(bls::launch_g1_decompress((const uint8_t*)a.sigs, a.n, (uint64_t*)c->d_xy.p, (int32_t*)c->d_st.p,
-                                     c->stream));
+        if (!decoded)
+            CK(bls::launch_g1_decompress((const uint8_t*)a.sigs, a.n, (uint64_t*)c->d_xy.p, (int32_t*)c->d_st.p,
+                                         c->stream));
         a.sig_xy = (const uint64_t*)c->d_xy.p;
         status = (const uint32_t*)c->d_st.p;
     }
@@ -439,9 +441,10 @@ int prepare(bls_ctx* c, size_t n, int fmt, bool want_ml, bool want_gt, bool stag
 
 // enqueue: staged inputs -> device, verify, results -> h_res (no synchronise);
 // nhms_on_device: d_nhms was filled on the device (a hash launch) instead;
-// inputs_on_device: the caller has already queued every input copy
+// inputs_on_device: the caller has already queued every input copy; decoded: and the
+// launch that decodes the signatures
 int enqueue(bls_ctx* c, size_t n, int fmt, bool persistent, bool want_ml, bool want_gt,
-            bool nhms_on_device = false, bool inputs_on_device = false) {
+            bool nhms_on_device = false, bool inputs_on_device = false, bool decoded = false) {
     size_t sig_bytes = n * (fmt == BLS_SIG_COMPRESSED ? 48 : 96);
     if (!inputs_on_device) {
         CK(cudaMemcpyAsync(c->d_sigs.p, c->h_sigs.p, sig_bytes, cudaMemcpyHostToDevice, c->stream));
@@ -465,14 +468,16 @@ int enqueue(bls_ctx* c, size_t n, int fmt, bool persistent, bool want_ml, bool w
     a.ml_out = want_ml ? (uint64_t*)c->d_ml.p : nullptr;
     a.gt_out = want_gt ? (uint64_t*)c->d_gt.p : nullptr;
     a.work_counter = persistent ? (int*)c->d_work.p : nullptr;
-    int rc = run_verify(c, a);
+    int rc = run_verify(c, a, decoded);
     if (rc) return rc;
     CK(cudaMemcpyAsync(c->h_res.p, a.results, n * 4, cudaMemcpyDeviceToHost, c->stream));
     return BLS_OK;
 }
 
-// messages + offsets + domain to the device, then -H(m_i) into d_nhms
-int stage_hash(bls_ctx* c, const uint8_t* msgs, const uint32_t* offsets, int n, const uint8_t* dst, int dst_len) {
+// messages + offsets + domain to the device, then -H(m_i) into d_nhms; decode: and
+// the n signatures of d_sigs into d_xy and d_st (grown by prepare)
+int stage_hash(bls_ctx* c, const uint8_t* msgs, const uint32_t* offsets, int n, const uint8_t* dst, int dst_len,
+               bool decode = false) {
     if (offsets[0] != 0) return fail(BLS_ERR_INVALID, "offsets[0] must be 0");
     for (int i = 0; i < n; ++i)
         if (offsets[i + 1] < offsets[i]) return fail(BLS_ERR_INVALID, "offsets decrease at %d", i);
@@ -484,8 +489,14 @@ int stage_hash(bls_ctx* c, const uint8_t* msgs, const uint32_t* offsets, int n, 
     if (bytes) CK(cudaMemcpyAsync(c->d_msg.p, msgs, bytes, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(c->d_off.p, offsets, ((size_t)n + 1) * 4, cudaMemcpyHostToDevice, c->stream));
     if (dst_len) CK(cudaMemcpyAsync(c->d_dst.p, dst, dst_len, cudaMemcpyHostToDevice, c->stream));
-    CK(bls::launch_neg_hash_to_g1((const uint8_t*)c->d_msg.p, (const uint32_t*)c->d_off.p, n,
-                                  (const uint8_t*)c->d_dst.p, dst_len, (uint64_t*)c->d_nhms.p, c->stream));
+    if (decode)
+        CK(bls::launch_neg_hash_decode((const uint8_t*)c->d_msg.p, (const uint32_t*)c->d_off.p, n,
+                                       (const uint8_t*)c->d_dst.p, dst_len, (uint64_t*)c->d_nhms.p,
+                                       (const uint8_t*)c->d_sigs.p, (uint64_t*)c->d_xy.p, (int32_t*)c->d_st.p,
+                                       c->stream));
+    else
+        CK(bls::launch_neg_hash_to_g1((const uint8_t*)c->d_msg.p, (const uint32_t*)c->d_off.p, n,
+                                      (const uint8_t*)c->d_dst.p, dst_len, (uint64_t*)c->d_nhms.p, c->stream));
     return BLS_OK;
 }
 
@@ -1254,8 +1265,10 @@ int bls_verify_messages(bls_ctx* ctx, int fmt, const void* sigs, const uint8_t* 
     CK(cudaMemcpyAsync(ctx->d_sigs.p, sigs, k * (fmt == BLS_SIG_COMPRESSED ? 48 : 96), cudaMemcpyHostToDevice,
                        ctx->stream));
     CK(cudaMemcpyAsync(ctx->d_pkidx.p, pk_ids, k * 4, cudaMemcpyHostToDevice, ctx->stream));
-    if ((rc = stage_hash(ctx, msgs, offsets, n, dst, dst_len))) return rc;
-    if ((rc = enqueue(ctx, k, fmt, false, false, false, true, true))) return rc;
+    // the thread-per-verification kernel decodes by itself
+    const bool decode = fmt == BLS_SIG_COMPRESSED && ctx->cfg.lanes_per_pairing != 1;
+    if ((rc = stage_hash(ctx, msgs, offsets, n, dst, dst_len, decode))) return rc;
+    if ((rc = enqueue(ctx, k, fmt, false, false, false, true, true, decode))) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
     memcpy(results, ctx->h_res.p, k * 4);
     return BLS_OK;

@@ -277,7 +277,7 @@ static __device__ __noinline__ bool quad_in_subgroup(const fp& x, const fp& y) {
     const bool ok = fp_eq(acc.X, bx) && fp_is_zero(fp_add(acc.Y, fp_mul_ool(y, Z3)));
     // a point of small order met an exceptional addition: one lane, all cases handled.
     // x = 0, the identity's encoding among them, is a point of order 3, outside without
-    // that second chain (448 encodings with an identity: 1.60 -> 0.59 ms).
+    // that second chain of 1 ms.
     return bad ? (!fp_is_zero(x) && g1_in_subgroup(x, y)) : (ok && !fp_is_zero(acc.Z));
 }
 
@@ -328,6 +328,54 @@ __device__ __forceinline__ int32_t g1_decode(const uint8_t* in, fp& x, fp& y, bo
 // the raw-ABI identity convention: x = 0 and y in {0, R mod p}
 __device__ __forceinline__ bool g1_limbs_identity(const fp& x, const fp& y) {
     return fp_is_zero(x) && (fp_is_zero(y) || fp_eq(y, fp_one()));
+}
+
+// point i, decoded by one thread with every check
+__device__ __forceinline__ void g1_decode_store(const uint8_t* in, int i, uint64_t* xy, int32_t* status) {
+    fp x, y;
+    bool id;
+    const int32_t st = g1_decode(in + 48 * (size_t)i, x, y, id, true);
+    status[i] = st;
+    fp_store_u64(xy + 12 * (size_t)i, x);
+    fp_store_u64(xy + 12 * (size_t)i + 6, y);
+}
+
+// Points base .. base + 15 of n by a block of three warps; inside: 16 bytes of
+// shared memory.  Warp 0 takes the square roots, a lane to a point; warps 1 and
+// 2 run the subgroup test, four lanes to a point (quad_in_subgroup), at the same
+// time.  The test does not need the root: with d = x^3 + 4 the point (d x, d^2)
+// lies on y^2 = x^3 + 4 d^3, and when d = y^2 the map (x, y) -> (y^2 x, y^3 y) takes the
+// curve to that one, (x, +-y) to (d x, d^2), and commutes with (x, y) -> (beta x, y),
+// while the doubling and addition formulas do not use the constant term.  When d
+// is not a square the point is off the curve and the test's answer is dropped.
+constexpr int kQuadPoints = 16, kQuadThreads = 96;
+__device__ __forceinline__ void g1_decode_quad(int base, const uint8_t* in, int n, uint64_t* xy, int32_t* status,
+                                               uint8_t* inside) {
+    const int t = threadIdx.x;
+    fp x, y;
+    bool id = false;
+    int32_t st = ST_OK;
+    const bool have = t < kQuadPoints && base + t < n;
+    if (t < 32) {
+        if (have) st = g1_decode(in + 48 * (size_t)(base + t), x, y, id, false);
+    } else {
+        const int j = (t - 32) >> 2;
+        // past the end: the last point again, so that the warp stays together
+        const int i = base + j < n ? base + j : n - 1;
+        const fp xm = fp_to_mont(g1_raw_x(in + 48 * (size_t)i));
+        const fp d = fp_add(fp_mul_ool(fp_sqr_ool(xm), xm), fp_four());
+        const bool ok = quad_in_subgroup(fp_mul_ool(d, xm), fp_sqr_ool(d));
+        if ((t & 3) == 0) inside[j] = ok ? 1 : 0;
+    }
+    __syncthreads();
+    if (!have) return;
+    if (st == ST_OK && !id && !inside[t]) {
+        st = ST_NOT_IN_SUBGROUP;
+        x = y = fp_zero();
+    }
+    status[base + t] = st;
+    fp_store_u64(xy + 12 * (size_t)(base + t), x);
+    fp_store_u64(xy + 12 * (size_t)(base + t) + 6, y);
 }
 
 }  // namespace bls

@@ -14,11 +14,10 @@ namespace bls {
 
 constexpr int kHashThreads = 64;
 
-__global__ void __launch_bounds__(kHashThreads) k_neg_hash_to_g1(const uint8_t* msgs, const uint32_t* offsets,
-                                                                 int n, const uint8_t* dst, int dst_len,
-                                                                 uint64_t* out) {
-    __shared__ uint4 xch[kHashThreads / 2][9];   // the odd thread's mapped point (Jacobian X, Y, Z)
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+// xch: the odd threads' mapped points (Jacobian X, Y, Z)
+__device__ __forceinline__ void neg_hash_block(int base, const uint8_t* msgs, const uint32_t* offsets, int n,
+                                               const uint8_t* dst, int dst_len, uint64_t* out, uint4 (*xch)[9]) {
+    const int t = 2 * base + threadIdx.x;
     const int i = t >> 1, which = t & 1;
     const bool live = i < n;
     g1j pt;
@@ -64,7 +63,33 @@ __global__ void __launch_bounds__(kHashThreads) k_neg_hash_to_g1(const uint8_t* 
     fp_store_u64(out + 12 * (size_t)i + 6, oy);
 }
 
-// The same for batches too small to fill the chip: eight lanes to a message, a
+__global__ void __launch_bounds__(kHashThreads) k_neg_hash_to_g1(const uint8_t* msgs, const uint32_t* offsets,
+                                                                 int n, const uint8_t* dst, int dst_len,
+                                                                 uint64_t* out) {
+    __shared__ uint4 xch[kHashThreads / 2][9];
+    neg_hash_block(blockIdx.x * (kHashThreads / 2), msgs, offsets, n, dst, dst_len, out, xch);
+}
+
+// The hashes of n messages and the decoded points of as many signatures in one
+// launch: blocks 0 .. hash_blocks - 1 hash, the others decode, a thread a point.  Two
+// latency chains of which neither reads what the other writes, on three warps an SM
+// for 4,736 of each.
+__global__ void __launch_bounds__(kHashThreads) k_neg_hash_decode_wide(const uint8_t* msgs, const uint32_t* offsets,
+                                                                      int n, const uint8_t* dst, int dst_len,
+                                                                      uint64_t* out, int hash_blocks,
+                                                                      const uint8_t* sigs, uint64_t* xy,
+                                                                      int32_t* status) {
+    __shared__ uint4 xch[kHashThreads / 2][9];
+    const int b = blockIdx.x;
+    if (b < hash_blocks) {
+        neg_hash_block(b * (kHashThreads / 2), msgs, offsets, n, dst, dst_len, out, xch);
+        return;
+    }
+    const int i = (b - hash_blocks) * kHashThreads + threadIdx.x;
+    if (i < n) g1_decode_store(sigs, i, xy, status);
+}
+
+// The hash for batches too small to fill the chip: eight lanes to a message, a
 // quad of four to each of its two field elements.  The quad's lanes map the element
 // together (the power is a chain that all four repeat), evaluate one polynomial of
 // the isogeny each, and the two quads exchange their points and clear the cofactor
@@ -72,12 +97,8 @@ __global__ void __launch_bounds__(kHashThreads) k_neg_hash_to_g1(const uint8_t* 
 // Bound by one dependent chain, for a 32-byte message in cycles: expansion 101 k,
 // the map with its power of 379 squarings 818 k, isogeny 108 k, sum and cofactor
 // 479 k, inverse 78 k.
-constexpr int kHashQuadThreads = 32;
-
-__global__ void __launch_bounds__(kHashQuadThreads) k_neg_hash_to_g1_quad(const uint8_t* msgs, const uint32_t* offsets,
-                                                                         int n, const uint8_t* dst, int dst_len,
-                                                                         uint64_t* out) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void neg_hash_quad(int t, const uint8_t* msgs, const uint32_t* offsets, int n,
+                                              const uint8_t* dst, int dst_len, uint64_t* out) {
     const int which = (t >> 2) & 1;
     const int i = t >> 3, m = i < n ? i : n - 1;     // past the end: the last message again, the warp stays together
     const uint32_t a = offsets[m], b = offsets[m + 1];
@@ -106,6 +127,27 @@ __global__ void __launch_bounds__(kHashQuadThreads) k_neg_hash_to_g1_quad(const 
     fp_store_u64(out + 12 * (size_t)i + 6, oy);
 }
 
+constexpr int kHashQuadThreads = 32;
+__global__ void __launch_bounds__(kHashQuadThreads) k_neg_hash_to_g1_quad(const uint8_t* msgs, const uint32_t* offsets,
+                                                                         int n, const uint8_t* dst, int dst_len,
+                                                                         uint64_t* out) {
+    neg_hash_quad(blockIdx.x * blockDim.x + threadIdx.x, msgs, offsets, n, dst, dst_len, out);
+}
+
+// The hashes and the decoded points of k_neg_hash_decode_wide in the small-batch forms:
+// hash blocks of three warps, four messages each, and g1_decode_quad's.
+__global__ void __launch_bounds__(kQuadThreads) k_neg_hash_decode(const uint8_t* msgs, const uint32_t* offsets, int n,
+                                                                 const uint8_t* dst, int dst_len, uint64_t* out,
+                                                                 int hash_blocks, const uint8_t* sigs, uint64_t* xy,
+                                                                 int32_t* status) {
+    __shared__ uint8_t inside[kQuadPoints];
+    const int b = blockIdx.x;
+    if (b >= hash_blocks)
+        g1_decode_quad((b - hash_blocks) * kQuadPoints, sigs, n, xy, status, inside);
+    else if (b * (kQuadThreads / 8) + (int)(threadIdx.x >> 5) * 4 < n)     // the warp has a message
+        neg_hash_quad(b * kQuadThreads + threadIdx.x, msgs, offsets, n, dst, dst_len, out);
+}
+
 // bls_neg_hash_to_g1 from host buffers, eight lanes against two: 1 message 0.84 and
 // 1.34 ms, 1,000 messages 0.87 and 1.37 ms, 2,368 (a warp on every scheduler) 0.88 and
 // 1.37 ms, 4,736 (two) 1.21 and 1.40 ms; 7,104 messages 1.87 against 1.42 ms.
@@ -122,6 +164,36 @@ cudaError_t launch_neg_hash_to_g1(const uint8_t* msgs, const uint32_t* offsets, 
     const long long threads = 2LL * n;
     k_neg_hash_to_g1<<<(unsigned)((threads + kHashThreads - 1) / kHashThreads), kHashThreads, 0, s>>>(
         msgs, offsets, n, dst, dst_len, out);
+    return cudaGetLastError();
+}
+
+// bls_verify_messages of compressed signatures from host buffers: the small-batch forms
+// in two launches, in one, and the thread-a-point forms in one.  1,000 items 3.94, 3.40
+// and 4.07 ms; 2,000 items 4.17, 3.95, 4.29 ms; 2,368 items, where the hash alone has a
+// warp on every scheduler, 4.18, 4.26, 4.29 ms; 3,000 items 5.37, 5.12, 5.01 ms; 4,736
+// items 5.44, 6.03, 5.04 ms (the eight- and four-lane forms repeat work, and side by side
+// that fills the chip).  Two launches of the thread-a-point forms, for more items than
+// the small-batch forms take: 14,208 items 13.69, in one 13.30 ms; 40,000 37.9 and 37.2 ms.
+constexpr int kHashDecodeQuadMax = 2072;    // 14 of each an SM
+constexpr int kHashDecodeTwoMax = 2368;     // 16
+
+cudaError_t launch_neg_hash_decode(const uint8_t* msgs, const uint32_t* offsets, int n, const uint8_t* dst,
+                                   int dst_len, uint64_t* out, const uint8_t* sigs, uint64_t* xy, int32_t* status,
+                                   cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    if (n <= kHashDecodeQuadMax) {
+        const int hash_blocks = (8 * n + kQuadThreads - 1) / kQuadThreads;
+        k_neg_hash_decode<<<hash_blocks + (n + kQuadPoints - 1) / kQuadPoints, kQuadThreads, 0, s>>>(
+            msgs, offsets, n, dst, dst_len, out, hash_blocks, sigs, xy, status);
+        return cudaGetLastError();
+    }
+    if (n <= kHashDecodeTwoMax) {
+        const cudaError_t e = launch_neg_hash_to_g1(msgs, offsets, n, dst, dst_len, out, s);
+        return e != cudaSuccess ? e : launch_g1_decompress(sigs, n, xy, status, s);
+    }
+    const int hash_blocks = (n + kHashThreads / 2 - 1) / (kHashThreads / 2);
+    k_neg_hash_decode_wide<<<hash_blocks + (n + kHashThreads - 1) / kHashThreads, kHashThreads, 0, s>>>(
+        msgs, offsets, n, dst, dst_len, out, hash_blocks, sigs, xy, status);
     return cudaGetLastError();
 }
 

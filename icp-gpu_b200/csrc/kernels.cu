@@ -58,57 +58,19 @@ __global__ void __launch_bounds__(kVerifyThreads) k_verify(VerifyArgs a) {
 }
 
 __global__ void __launch_bounds__(128) k_g1_decompress(const uint8_t* in, int n, uint64_t* xy, int32_t* status) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    fp x, y;
-    bool id;
-    int32_t st = g1_decode(in + 48 * (size_t)i, x, y, id, true);
-    status[i] = st;
-    fp_store_u64(xy + 12 * (size_t)i, x);
-    fp_store_u64(xy + 12 * (size_t)i + 6, y);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) g1_decode_store(in, i, xy, status);
 }
 
-// The same decode for batches too small to fill the chip: a block of three warps
-// takes 16 points.  Warp 0 takes the square roots, a lane to a point; warps 1 and
-// 2 run the subgroup test, four lanes to a point (quad_in_subgroup), at the same
-// time.  The test does not need the root: with d = x^3 + 4 the point (d x, d^2)
-// lies on y^2 = x^3 + 4 d^3, and when d = y^2 the map (x, y) -> (y^2 x, y^3 y) takes the
-// curve to that one, (x, +-y) to (d x, d^2), and commutes with (x, y) -> (beta x, y),
-// while the doubling and addition formulas do not use the constant term.  When d
-// is not a square the point is off the curve and the test's answer is dropped.
-// Bound by the latency of the subgroup chain (127 doublings and 16 additions), the
-// root's running beside it.  bls_g1_decompress_status from host buffers, this
-// form against a thread a point: 1 point 0.55 and 1.58 ms, 448 points 0.59 and
-// 1.61 ms, 2,368 points (a block on every SM) 0.66 and 1.66 ms.
-constexpr int kQuadPoints = 16, kQuadThreads = 96;
+// The same decode for batches too small to fill the chip, four lanes to a point
+// (g1_decode_quad).  Bound by the latency of the subgroup chain (127 doublings and 16
+// additions), the root's running beside it.  bls_g1_decompress_status from host
+// buffers, this form against a thread a point: 1 point 0.55 and 1.58 ms, 448 points
+// 0.59 and 1.61 ms, 2,368 points (a block on every SM) 0.66 and 1.66 ms.
 __global__ void __launch_bounds__(kQuadThreads) k_g1_decompress_quad(const uint8_t* in, int n, uint64_t* xy,
                                                                     int32_t* status) {
     __shared__ uint8_t inside[kQuadPoints];
-    const int base = blockIdx.x * kQuadPoints, t = threadIdx.x;
-    fp x, y;
-    bool id = false;
-    int32_t st = ST_OK;
-    const bool have = t < kQuadPoints && base + t < n;
-    if (t < 32) {
-        if (have) st = g1_decode(in + 48 * (size_t)(base + t), x, y, id, false);
-    } else {
-        const int j = (t - 32) >> 2;
-        // past the end: the last point again, so that the warp stays together
-        const int i = base + j < n ? base + j : n - 1;
-        const fp xm = fp_to_mont(g1_raw_x(in + 48 * (size_t)i));
-        const fp d = fp_add(fp_mul_ool(fp_sqr_ool(xm), xm), fp_four());
-        const bool ok = quad_in_subgroup(fp_mul_ool(d, xm), fp_sqr_ool(d));
-        if ((t & 3) == 0) inside[j] = ok ? 1 : 0;
-    }
-    __syncthreads();
-    if (!have) return;
-    if (st == ST_OK && !id && !inside[t]) {
-        st = ST_NOT_IN_SUBGROUP;
-        x = y = fp_zero();
-    }
-    status[base + t] = st;
-    fp_store_u64(xy + 12 * (size_t)(base + t), x);
-    fp_store_u64(xy + 12 * (size_t)(base + t) + 6, y);
+    g1_decode_quad(blockIdx.x * kQuadPoints, in, n, xy, status, inside);
 }
 
 // The serving ring's decoder: the same decode, grid-stride, in blocks that
