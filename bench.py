@@ -41,11 +41,13 @@ N_KEYS = 40
 SEED = 2
 METRIC = "BLS12-381 verifies/s, batched vs plain launch, bit-exact; serve p50/p99 ms"
 
-# Multiply instructions per verification in this implementation (the
-# six-lane kernels' generated op sequence, counted by gen_fp2ops.py over the
-# 646 programs of one verification): 20,684 products of 12 x 12 limbs, each by
-# one level of limb Karatsuba (three 6 x 6 products: 216 mul.lo / mul.hi), and
-# 7,284 Montgomery reductions (12 rows x 25) = 6,652,944.
+# Multiplies per verification of the generated op sequence in its half-coefficient
+# form (the five-item kernel's; counted by gen_fp2ops.py over the 646 programs of
+# one verification): 20,684 products of 12 x 12 limbs, each by one level of limb
+# Karatsuba (three 6 x 6 products: 108 pairs of mul.lo and mul.hi, 216 multiplies),
+# and 7,284 Montgomery reductions (12 rows of 12 pairs and one mul.lo, 300) =
+# 6,652,944.  The twelve-warp kernel's paired-warp form of the same programs has
+# 19,868 products.
 OWN_PRODUCTS_PER_VERIFY = 20684
 OWN_REDC_PER_VERIFY = 7284
 IMAD_PER_VERIFY = OWN_PRODUCTS_PER_VERIFY * 216 + OWN_REDC_PER_VERIFY * 300
@@ -437,21 +439,23 @@ def run_gpu(args):
             "kernel_ms": round(kernel_ms, 4),
             "chain_ceiling": round(chain_timad, 3),
             "frac_of_chain_ceiling": round(achieved_timad / chain_timad, 4),
-            "chain_ceiling_basis": "measured: 12 x 12-limb carry-chain products (288 IMAD each) in a loop with the "
-                                   "verify kernel's block shape and occupancy (bls_imad_chain_rate)",
+            "chain_ceiling_basis": "measured: schoolbook 12 x 12-limb products on paired columns (288 IMAD each) in a "
+                                   "loop with the five-item kernel's block shape and occupancy "
+                                   "(bls_imad_chain_rate)",
             # The nominal peak counts every IMAD at the full rate, but only the
             # low-word multiply issues at that rate: the high word (mul.hi /
-            # mul.wide) is measured at half of it.  The reference's CIOS
-            # multiply (and this kernel's products) are half low-word and half
-            # high-word multiplies, so the most the pipe can retire of that mix is
-            # the harmonic mean of the two rates.
+            # mul.wide) is measured at half of it.  Separate low-word and
+            # high-word multiplies, half of each, retire at most at the harmonic
+            # mean of the two rates.  The kernels' products write both multiply-adds
+            # of a pair of limbs next to each other, which issue as one 64-bit
+            # multiply-add, so they can exceed that mean.
             "imad_lo_rate": round(lo_rate / 1e12, 3),
             "imad_hi_rate": round(hi_rate / 1e12, 3),
             "mix_peak": round(2.0 / (1e12 / lo_rate + 1e12 / hi_rate), 3),
             "frac_of_mix_peak": round(achieved_timad / (2.0 / (1e12 / lo_rate + 1e12 / hi_rate)), 4),
             "mix_peak_basis": "measured (bls_imad_pipe_rates): independent mad.lo.u32 and mad.hi.u32 with every "
-                              "latency covered; a half-low, half-high multiply mix retires at most at their "
-                              "harmonic mean",
+                              "latency covered; separate low and high multiplies, half of each, retire at most at "
+                              "their harmonic mean; pairs of both on the same operands issue as one and can exceed it",
         }
         if full_chip:
             fc_timad = ALGO_IMAD_PER_VERIFY * full_chip["items"] / (full_chip["kernel_ms"] / 1e3) / 1e12
@@ -649,7 +653,7 @@ def run_batching(G, WL, ctx, wl_headline, reps=2):
     # the limb-layout dimension: product throughput of each layout in the
     # twelve-warp kernel's setting (bls_limb_layout_rates); the verify kernels
     # are built for the first, and the sweep shows whether it is still the fastest
-    layouts = ["12 x 32-bit limbs, limb Karatsuba, carry-chain rows (216 multiplies)",
+    layouts = ["12 x 32-bit limbs, limb Karatsuba, rows of paired multiply-adds (108 pairs)",
                "15 x 26-bit signed limbs, 225 mad.wide.s32 into 64-bit columns",
                "14 x 28-bit limbs, 196 mad.wide.u32 into 64-bit columns"]
     lpts = [{"layout": nm, "g_products_per_s": round(r / 1e9, 2)} for nm, r in zip(layouts, layout_rates)]

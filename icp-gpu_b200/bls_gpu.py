@@ -406,7 +406,7 @@ class Context:
         return res
 
     def imad_chain_rate(self):
-        """IMAD-pipe instructions/s of the carry-chain product loop (bls_imad_chain_rate)."""
+        """IMAD-pipe instructions/s of the paired-column product loop (bls_imad_chain_rate)."""
         v = ctypes.c_double(0.0)
         self._check(self.lib.bls_imad_chain_rate(self.h, ctypes.byref(v)), "bls_imad_chain_rate")
         return v.value
@@ -419,7 +419,7 @@ class Context:
 
     def limb_layout_rates(self):
         """Products/s of the three limb layouts in the verify kernel's setting
-        (bls_limb_layout_rates): [12 x 32-bit Karatsuba carry chains,
+        (bls_limb_layout_rates): [12 x 32-bit Karatsuba paired rows,
         15 x 26-bit signed wide columns, 14 x 28-bit wide columns]."""
         v = (ctypes.c_double * 3)()
         self._check(self.lib.bls_limb_layout_rates(self.h, v, 3), "bls_limb_layout_rates")

@@ -746,7 +746,7 @@ VerifyArgs items_from(VerifyArgs a, int first) {
 }  // namespace
 
 // As many lanes to an item as still give every item a place in one wave: four up
-// to 8 items a SM, two up to 16.  One launch of a block on every SM takes 3.50 ms
+// to 8 items a SM, two up to 16.  One launch of a block on every SM takes 3.47 ms
 // with a lane to an item, 2.77 ms with two and 2.51 ms with four (the sums shrink
 // from 2, 3, 5 and 9 products in the cyclotomic square, the line, the square and the
 // product to 1, 2, 3 and 5, or 1, 1, 2 and 3; the reductions stay).  A batch of

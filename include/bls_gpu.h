@@ -231,22 +231,24 @@ int bls_autotune(bls_ctx* ctx, const bls_batch* sample_device, int repeats, bls_
                  int max_points, int* n_points);
 
 /* Measured ceiling for the roofline: IMAD-pipe instructions per second of a
- * loop of 12 x 12-limb carry-chain products (the verify kernel's multiply
- * form: mul.lo / mul.hi chained through the carry flag) with the verify
- * kernel's block shape and occupancy, on the whole device. */
+ * loop of 12 x 12-limb products (the verify kernels' multiply form: pairs of
+ * mul.lo and mul.hi on the same operands, chained through the carry flag and
+ * counted as two) with the five-item kernel's block shape and occupancy, on the
+ * whole device. */
 int bls_imad_chain_rate(bls_ctx* ctx, double* imad_per_s);
 /* Measured issue rates of the two halves of a 32 x 32-bit product on the
  * whole device, in thread instructions per second: mul.lo (the low word) and
  * mul.hi (the high word), each from independent multiply-adds with every
- * latency covered.  Their ratio shows how far a multiprecision multiply, half
- * of whose multiplies are high words, can go toward the nominal IMAD peak. */
+ * latency covered.  Their harmonic mean bounds a multiprecision multiply of
+ * separate low-word and high-word chains; adjacent pairs on the same operands
+ * issue as one multiply and are not bound by it. */
 int bls_imad_pipe_rates(bls_ctx* ctx, double* lo_per_s, double* hi_per_s);
 /* The autotuner's limb-layout dimension: products per second on the whole
  * device of three layouts of a 381-bit element, each in the twelve-warp verify
  * kernel's setting (one block of 384 threads per SM, operands loaded from
  * lane-interleaved shared memory, every product accumulated):
- *   [0] 12 x 32-bit limbs, limb Karatsuba with carry-chain rows into a
- *       26-limb accumulator (the layout every verify kernel is built for),
+ *   [0] 12 x 32-bit limbs, limb Karatsuba with rows of paired multiply-adds
+ *       into a 26-limb accumulator (the layout every verify kernel is built for),
  *   [1] 15 x 26-bit signed limbs, 225 mad.wide.s32 into 64-bit columns,
  *   [2] 14 x 28-bit limbs, 196 mad.wide.u32 into 64-bit columns.
  * n_layouts must be at least BLS_LIMB_LAYOUTS. */
