@@ -155,6 +155,8 @@ struct bls_ctx {
     int sms = 0;
     std::mutex mu;
     size_t dev_bytes = 0;  // bytes held on the device by this context
+    bls::ChipUse use;      // this context among the calls at work on the device
+    cudaEvent_t ev_use = nullptr;   // after the work of a call that returns before it has run
 
     struct DevBuf {
         void* p = nullptr;
@@ -299,6 +301,8 @@ struct bls_ctx {
         graph_key.clear();
     }
     void release() {
+        use.end();
+        if (ev_use) cudaEventDestroy(ev_use);
         drop_graph();
         for (DevBuf* b : {&d_sigs, &d_nhms, &d_pkidx, &d_res, &d_ml, &d_gt, &d_pk_items, &d_g2_call, &d_in,
                           &d_xy, &d_st, &d_work, &d_msg, &d_off, &d_dst, &d_rlc})
@@ -337,6 +341,7 @@ int ctx_init(bls_ctx* c, const bls_config* cfg) {
     CK(cudaSetDevice(c->cfg.device));
     CK(cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->cfg.device));
     CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
+    CK(cudaEventCreateWithFlags(&c->ev_use, cudaEventDisableTiming));
     size_t pk_bytes = (size_t)c->cfg.max_pks * bls::kCoeffU64 * 8;
     size_t norm_bytes = pk_bytes + bls::kCoeffU64 * 8 + (size_t)(c->cfg.max_pks + 1) * (12 * 8 + 1);
     size_t need = pk_bytes + c->cfg.max_pks + bls::kCoeffU64 * 8 + 24 * 8 + norm_bytes;
@@ -392,6 +397,35 @@ int default_ctx(bls_ctx** out) {
     return BLS_OK;
 }
 
+// A call of the context that launches verify kernels, counted on its device until it
+// returns; or, after left_running, until what its stream holds then has run.
+class Working {
+  public:
+    explicit Working(bls_ctx* c) : c_(c) { c->use.begin(c->cfg.device, c->sms); }
+    ~Working() {
+        if (c_) c_->use.end();
+    }
+    int left_running() {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        CK(cudaStreamIsCapturing(c_->stream, &st));
+        if (st != cudaStreamCaptureStatusNone) return BLS_OK;   // nothing runs yet
+        CK(cudaEventRecord(c_->ev_use, c_->stream));
+        c_->use.end_when(bls::event_done, c_->ev_use);
+        c_ = nullptr;
+        return BLS_OK;
+    }
+
+  private:
+    bls_ctx* c_;
+};
+
+// lanes to an item of a verify of n items (0 where the kernel has one form only)
+int plan_lanes(bls_ctx* c, int n) {
+    return c->cfg.lanes_per_pairing == 6 && bls::six_lane_shape(c->cfg.threads_per_block) == bls::kShapeWide
+               ? c->use.plan_verify(n)
+               : 0;
+}
+
 // One verify launch on the context stream.  lanes_per_pairing 1 runs the
 // thread-per-verification kernel (which decodes compressed signatures itself);
 // otherwise compressed signatures are first decoded into scratch buffers by
@@ -416,6 +450,7 @@ int run_verify(bls_ctx* c, bls::VerifyArgs a, bool decoded = false) {
         status = (const uint32_t*)c->d_st.p;
     }
     if (a.work_counter) CK(cudaMemsetAsync(a.work_counter, 0, sizeof(int), c->stream));
+    if (!a.item_lanes) a.item_lanes = plan_lanes(c, a.n);
     CK(bls::launch_verify_lanes(a, status, c->cfg.lanes_per_pairing, c->cfg.threads_per_block, c->cfg.blocks_per_sm,
                                 c->sms, c->stream));
     return BLS_OK;
@@ -442,9 +477,9 @@ int prepare(bls_ctx* c, size_t n, int fmt, bool want_ml, bool want_gt, bool stag
 // enqueue: staged inputs -> device, verify, results -> h_res (no synchronise);
 // nhms_on_device: d_nhms was filled on the device (a hash launch) instead;
 // inputs_on_device: the caller has already queued every input copy; decoded: and the
-// launch that decodes the signatures
+// launch that decodes the signatures; item_lanes: as planned already (0: planned here)
 int enqueue(bls_ctx* c, size_t n, int fmt, bool persistent, bool want_ml, bool want_gt,
-            bool nhms_on_device = false, bool inputs_on_device = false, bool decoded = false) {
+            bool nhms_on_device = false, bool inputs_on_device = false, bool decoded = false, int item_lanes = 0) {
     size_t sig_bytes = n * (fmt == BLS_SIG_COMPRESSED ? 48 : 96);
     if (!inputs_on_device) {
         CK(cudaMemcpyAsync(c->d_sigs.p, c->h_sigs.p, sig_bytes, cudaMemcpyHostToDevice, c->stream));
@@ -468,6 +503,7 @@ int enqueue(bls_ctx* c, size_t n, int fmt, bool persistent, bool want_ml, bool w
     a.ml_out = want_ml ? (uint64_t*)c->d_ml.p : nullptr;
     a.gt_out = want_gt ? (uint64_t*)c->d_gt.p : nullptr;
     a.work_counter = persistent ? (int*)c->d_work.p : nullptr;
+    a.item_lanes = item_lanes;
     int rc = run_verify(c, a, decoded);
     if (rc) return rc;
     CK(cudaMemcpyAsync(c->h_res.p, a.results, n * 4, cudaMemcpyDeviceToHost, c->stream));
@@ -857,6 +893,7 @@ int bls_verify_batch(bls_ctx* ctx, const bls_batch* b, int32_t* results) {
     int rc;
     if ((rc = check_ids(ctx, b->pk_ids, b->n))) return rc;
     CK(cudaSetDevice(ctx->cfg.device));
+    Working call(ctx);
     size_t n = (size_t)b->n;
     size_t sig_bytes = n * (b->sig_format == BLS_SIG_COMPRESSED ? 48 : 96);
     if ((rc = prepare(ctx, n, b->sig_format, b->miller_out != nullptr, b->gt_out != nullptr, false))) return rc;
@@ -894,6 +931,7 @@ int bls_verify_requests(bls_ctx* ctx, const bls_request* reqs, int nreq, int fmt
     for (int r = 0; r < nreq; ++r)
         if ((rc = check_ids(ctx, reqs[r].pk_ids, reqs[r].n))) return rc;
     CK(cudaSetDevice(ctx->cfg.device));
+    Working call(ctx);
     const size_t sb = fmt == BLS_SIG_COMPRESSED ? 48 : 96;
     if (mode == BLS_MODE_PLAIN) {
         for (int r = 0; r < nreq; ++r) {
@@ -919,6 +957,7 @@ int bls_verify_requests(bls_ctx* ctx, const bls_request* reqs, int nreq, int fmt
         memcpy((char*)ctx->h_nhms.p + at * 96, reqs[r].neg_hms, n * 96);
         memcpy((char*)ctx->h_pkidx.p + at * 4, reqs[r].pk_ids, n * 4);
     });
+    const int item_lanes = plan_lanes(ctx, (int)total);
     std::vector<const void*> key = {(const void*)total, (const void*)(size_t)fmt,
                                     (const void*)(size_t)ctx->cfg.lanes_per_pairing,
                                     (const void*)(size_t)ctx->cfg.threads_per_block,
@@ -926,14 +965,15 @@ int bls_verify_requests(bls_ctx* ctx, const bls_request* reqs, int nreq, int fmt
                                     ctx->d_pkidx.p, ctx->d_res.p, ctx->d_work.p, ctx->d_xy.p, ctx->d_st.p,
                                     ctx->h_sigs.p, ctx->h_nhms.p, ctx->h_pkidx.p, ctx->h_res.p,
                                     // the key count the kernel checks ids against, and the table form
-                                    (const void*)(size_t)ctx->n_pks, (const void*)(size_t)ctx->norm_ok};
+                                    (const void*)(size_t)ctx->n_pks, (const void*)(size_t)ctx->norm_ok,
+                                    (const void*)(size_t)item_lanes};
     if (!ctx->graph || ctx->graph_key != key) {
         ctx->drop_graph();
         if (ctx->cfg.lanes_per_pairing > 1)   // set up outside capture
             bls::verify_lanes_blocks_per_sm(ctx->cfg.lanes_per_pairing, ctx->cfg.threads_per_block);
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-        rc = enqueue(ctx, total, fmt, true, false, false);
+        rc = enqueue(ctx, total, fmt, true, false, false, false, false, false, item_lanes);
         cudaError_t ec = cudaStreamEndCapture(ctx->stream, &g);
         if (rc) {
             if (g) cudaGraphDestroy(g);
@@ -992,6 +1032,7 @@ int bls_autotune(bls_ctx* ctx, const bls_batch* b, int repeats, bls_tune_point* 
     if (repeats <= 0) repeats = 3;
     std::lock_guard<std::mutex> lk(ctx->mu);
     CK(cudaSetDevice(ctx->cfg.device));
+    Working call(ctx);
     int rc;
     if ((rc = ctx->grow(ctx->d_res, (size_t)b->n * 4)) || (rc = ctx->grow(ctx->d_work, 256))) return rc;
     if (b->sig_format == BLS_SIG_COMPRESSED &&
@@ -1088,7 +1129,9 @@ int bls_verify_batch_device(bls_ctx* ctx, const bls_batch* b, int32_t* results_d
     a.results = results_device;
     a.ml_out = b->miller_out;
     a.gt_out = b->gt_out;
-    return run_verify(ctx, a);
+    Working call(ctx);
+    if (int rc = run_verify(ctx, a)) return rc;
+    return call.left_running();
 }
 
 // Random-linear-combination batch: see rlc.cu.  Host side: scalars, the items
@@ -1128,6 +1171,7 @@ int bls_verify_batch_rlc(bls_ctx* ctx, const bls_batch* b, const uint64_t* scala
     int rc;
     if ((rc = check_ids(ctx, b->pk_ids, b->n))) return rc;
     CK(cudaSetDevice(ctx->cfg.device));
+    Working call(ctx);
     // items grouped by key; key slots in increasing id; tiles of one key
     std::vector<int32_t> start(ctx->n_pks + 1, 0), order(n), keys, key_tile, tiles;
     for (size_t i = 0; i < n; ++i) start[b->pk_ids[i] + 1]++;
@@ -1260,6 +1304,7 @@ int bls_verify_messages(bls_ctx* ctx, int fmt, const void* sigs, const uint8_t* 
     std::lock_guard<std::mutex> lk(ctx->mu);
     if ((rc = check_ids(ctx, pk_ids, n))) return rc;
     CK(cudaSetDevice(ctx->cfg.device));
+    Working call(ctx);
     const size_t k = (size_t)n;
     if ((rc = prepare(ctx, k, fmt, false, false, false))) return rc;
     CK(cudaMemcpyAsync(ctx->d_sigs.p, sigs, k * (fmt == BLS_SIG_COMPRESSED ? 48 : 96), cudaMemcpyHostToDevice,
@@ -1405,6 +1450,7 @@ int gpu_batch_bls_verify(const uint64_t* sigs, const uint64_t* neg_hms, const ui
     std::lock_guard<std::mutex> lk(c->mu);
     auto body = [&]() -> int {
         CK(cudaSetDevice(c->cfg.device));
+        Working call(c);
         size_t n = (size_t)M;
         const size_t W = bls::kCoeffU64;
         bool done = false;

@@ -3,6 +3,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "chip_share.h"
+
 namespace bls {
 
 constexpr int kVerifyThreads = 64;
@@ -27,6 +29,9 @@ struct VerifyArgs {
     uint64_t* gt_out;            // n x 72 or NULL, device
     const uint64_t* sig_xy;      // decoded signatures (n x 12 u64) when sigs were compressed, device
     int* work_counter;           // persistent mode: items are claimed from this zeroed counter, device
+    // k_verify_w: lanes to an item in the wave that n does not fill (ChipUse::plan_verify);
+    // 0 = as if the launch had the whole chip
+    int item_lanes;
     // Normalised line tables (every row divided by its c2) and the Miller
     // correction factors (Fp2, 12 u64) of the generator and the keys, device;
     // pk_norm NULL = use the raw tables.  Read by the Fp2-lane kernel only.
@@ -103,6 +108,17 @@ cudaError_t launch_lines_normalize(const uint64_t* raw, int n, uint64_t* norm, u
 constexpr int kShapeFive = 64, kShapeWide = 384;
 constexpr int kDefaultShape = kShapeWide;
 inline int six_lane_shape(int threads_per_block) { return threads_per_block > 0 ? threads_per_block : kDefaultShape; }
+
+// whether the work that an event was recorded after has run (ChipUse::end_when); asked
+// while some stream of the process may be in a capture, which a plain query would end
+inline bool event_done(const void* event) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = cudaEventQuery((cudaEvent_t) const_cast<void*>(event));
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e == cudaErrorNotReady && cudaPeekAtLastError() == cudaErrorNotReady) cudaGetLastError();
+    return e != cudaErrorNotReady;
+}
 
 // lane-parallel verify; in_status: per-item decode status or NULL.  lanes 6
 // runs an Fp2-lane kernel of block shape `shape` (verify_fp2.cu or

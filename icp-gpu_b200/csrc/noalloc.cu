@@ -22,11 +22,12 @@
 //     two calls whose work overlaps on the GPU (different streams, no ordering
 //     between them) race on the array and produce wrong results;
 //   * the first call on a device does the set-up: it resolves the array's
-//     device address (cudaGetSymbolAddress, with that device current) and
+//     device address (cudaGetSymbolAddress, with that device current), makes
+//     the event that tells when a call's work has run (chip_share.h) and
 //     sets the verify kernel's shared-memory attribute; make that first call
-//     before starting any stream capture.  The address is cached per device
+//     before starting any stream capture.  Address and event are kept per device
 //     ordinal for the life of the process; after cudaDeviceReset the module is
-//     loaded again and the cached address is stale, so this entry point must
+//     loaded again and both are stale, so this entry point must
 //     not be used across a device reset.
 #include <cuda_runtime.h>
 
@@ -48,21 +49,29 @@ constexpr size_t kScratchBytes = kXyBytes + kStatusBytes + kIndexBytes + kCounte
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
 constexpr int kMaxDevices = 64;
-std::mutex g_mu;
-unsigned char* g_addr[kMaxDevices] = {};
+// Per device: the scratch array's address, and the calls' use of the chip, which ends
+// when the event behind the last call's work has passed (the calls of a device are
+// ordered, so one use stands for them).  Never destroyed: an exiting process's driver may be gone.
+struct PerDevice {
+    std::mutex mu;
+    unsigned char* addr = nullptr;
+    cudaEvent_t ran = nullptr;
+    ChipUse use;
+};
+PerDevice& per_device(int dev) {
+    static PerDevice* all = new PerDevice[kMaxDevices];
+    return all[dev];
+}
 
-// device address of the scratch array on the current device (set up once)
-cudaError_t scratch_address(int dev, unsigned char** out) {
-    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
-    std::lock_guard<std::mutex> lk(g_mu);
-    if (!g_addr[dev]) {
-        void* p = nullptr;
-        cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-        if (e != cudaSuccess) return e;
-        g_addr[dev] = static_cast<unsigned char*>(p);
-    }
-    *out = g_addr[dev];
-    return cudaSuccess;
+// set up once, with the device current
+cudaError_t set_up(PerDevice& d) {
+    std::lock_guard<std::mutex> lk(d.mu);
+    if (d.addr) return cudaSuccess;
+    void* p = nullptr;
+    cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
+    if (e == cudaSuccess && !d.ran) e = cudaEventCreateWithFlags(&d.ran, cudaEventDisableTiming);
+    if (e == cudaSuccess) d.addr = static_cast<unsigned char*>(p);
+    return e;
 }
 
 // Item i's key index into the scratch copy: the caller's index when it names
@@ -98,8 +107,10 @@ extern "C" int bls_verify_compressed_noalloc(const uint8_t* sigs48, const uint64
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return BLS_ERR_CUDA;
-    unsigned char* base = nullptr;
-    if (bls::scratch_address(dev, &base) != cudaSuccess) return BLS_ERR_CUDA;
+    if (dev < 0 || dev >= bls::kMaxDevices) return BLS_ERR_CUDA;
+    bls::PerDevice& d = bls::per_device(dev);
+    if (bls::set_up(d) != cudaSuccess) return BLS_ERR_CUDA;
+    unsigned char* base = d.addr;
     uint64_t* xy = reinterpret_cast<uint64_t*>(base);
     int32_t* status = reinterpret_cast<int32_t*>(base + bls::kXyBytes);
     int32_t* idx = reinterpret_cast<int32_t*>(base + bls::kXyBytes + bls::kStatusBytes);
@@ -120,8 +131,17 @@ extern "C" int bls_verify_compressed_noalloc(const uint8_t* sigs48, const uint64
     a.n = n;
     a.results = results;
     a.work_counter = counter;
-    if (bls::launch_verify_lanes(a, reinterpret_cast<const uint32_t*>(status), lanes_per_pairing, 0, 0, sms, s) !=
-        cudaSuccess)
-        return BLS_ERR_CUDA;
-    return BLS_OK;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) return BLS_ERR_CUDA;
+    std::lock_guard<std::mutex> lk(d.mu);
+    d.use.begin(dev, sms);
+    if (lanes_per_pairing == 6) a.item_lanes = d.use.plan_verify(n);
+    const bool ok = bls::launch_verify_lanes(a, reinterpret_cast<const uint32_t*>(status), lanes_per_pairing, 0, 0, sms,
+                                             s) == cudaSuccess;
+    // a captured call runs nothing yet
+    if (ok && capture == cudaStreamCaptureStatusNone && cudaEventRecord(d.ran, s) == cudaSuccess)
+        d.use.end_when(bls::event_done, d.ran);
+    else
+        d.use.end();
+    return ok ? BLS_OK : BLS_ERR_CUDA;
 }

@@ -78,6 +78,7 @@ struct Slot {
     void *d_sigs = nullptr, *d_nhms = nullptr, *d_ids = nullptr, *d_res = nullptr, *d_xy = nullptr,
          *d_st = nullptr, *d_work = nullptr;
     bool busy = false;
+    bls::ChipUse use;   // from launch to finish
     std::vector<Pending> reqs;
 };
 
@@ -113,6 +114,7 @@ struct Ring {
     cudaStream_t copy = nullptr, kern = nullptr;
     cudaStream_t poll = nullptr;           // result reads, apart from the copy stream's decodes
     cudaEvent_t done = nullptr;
+    bls::ChipUse use;                      // while the ring's kernel is on the device
     // Publications do not wait: round r copies its count from its own pinned
     // word (h_pubv[r % kPubSlots]) and records pub_ev[r % kPubSlots] after the
     // copy; `confirmed` is the count of the newest publication known to have
@@ -174,6 +176,7 @@ struct bls_server {
             n += r.n;
         }
         cudaStream_t st = s.stream;
+        s.use.begin(view.device, view.sms);
         if (cudaMemcpyAsync(s.d_sigs, s.h_sigs, n * sb, cudaMemcpyHostToDevice, st) ||
             cudaMemcpyAsync(s.d_nhms, s.h_nhms, n * 96, cudaMemcpyHostToDevice, st) ||
             cudaMemcpyAsync(s.d_ids, s.h_ids, n * 4, cudaMemcpyHostToDevice, st) ||
@@ -202,6 +205,7 @@ struct bls_server {
             status = (const uint32_t*)s.d_st;
         }
         int lanes = view.lanes > 1 ? view.lanes : 6;
+        if (lanes == 6 && view.shape == bls::kShapeWide) a.item_lanes = s.use.plan_verify(a.n, false);
         if (bls::launch_verify_lanes(a, status, lanes, view.shape, view.blocks_per_sm, view.sms, st) ||
             cudaMemcpyAsync(s.h_res, s.d_res, n * 4, cudaMemcpyDeviceToHost, st) || cudaEventRecord(s.done, st))
             return BLS_ERR_CUDA;
@@ -221,6 +225,7 @@ struct bls_server {
         }
         items += off;
         s.reqs.clear();
+        s.use.end();
         s.busy = false;
     }
 
@@ -256,6 +261,9 @@ struct bls_server {
                                   ? bls::launch_verify_w_serve(a, st, blocks, view.sms, ring.kern)
                                   : bls::launch_verify_fp2_serve(a, st, blocks, view.sms, ring.kern);
         if (e != cudaSuccess || cudaEventRecord(ring.done, ring.kern) != cudaSuccess) return BLS_ERR_CUDA;
+        ring.use.begin(view.device, view.sms);
+        if (view.shape == bls::kShapeWide) ring.use.hold(blocks < view.sms ? blocks : view.sms);
+        ring.use.end_when(bls::event_done, ring.done);
         ring.launched = true;
         return BLS_OK;
     }
@@ -545,6 +553,7 @@ struct bls_server {
                 if (s.reqs.empty()) continue;
                 int rc = launch(s);
                 if (rc) {
+                    for (auto& x : slots) x.use.end();
                     error = rc;
                     cv_done.notify_all();
                     return;
@@ -648,7 +657,7 @@ int bls_server_create(bls_ctx* ctx, const bls_server_config* cfg, bls_server** o
         return BLS_ERR_NOMEM;
     }
     if (s->cfg.slots > admitted) s->cfg.slots = admitted;
-    s->slots.resize(s->cfg.slots);
+    s->slots = std::vector<Slot>(s->cfg.slots);
     for (auto& sl : s->slots) {
         bool ok = cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking) == cudaSuccess &&
                   cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming) == cudaSuccess &&
@@ -697,12 +706,14 @@ void bls_server_destroy(bls_server* s) {
         for (void* p : {(void*)r.d_sigs, (void*)r.d_nhms, (void*)r.d_ids, (void*)r.d_res, (void*)r.d_ctl,
                         (void*)r.d_comp, (void*)r.d_st, (void*)r.d_sub})
             if (p) cudaFree(p);
+        r.use.end();
         if (r.done) cudaEventDestroy(r.done);
         if (r.copy) cudaStreamDestroy(r.copy);
         if (r.kern) cudaStreamDestroy(r.kern);
     }
     for (auto& sl : s->slots) {
         if (sl.stream) cudaStreamSynchronize(sl.stream);
+        sl.use.end();
         for (void* p : {sl.h_sigs, sl.h_nhms, sl.h_ids, sl.h_res})
             if (p) cudaFreeHost(p);
         for (void* p : {sl.d_sigs, sl.d_nhms, sl.d_ids, sl.d_res, sl.d_xy, sl.d_st, sl.d_work})

@@ -40,7 +40,7 @@
 namespace bls {
 namespace {
 
-constexpr int kV = 32;                           // items a block holds at most, one per lane
+constexpr int kV = kBlockItems;                  // items a block holds at most, one per lane
 constexpr int kRoles = 12;                       // warps per block
 constexpr int kThreads = 32 * kRoles;
 constexpr int kGroups = f2::kGroupsUsed;
@@ -745,20 +745,19 @@ VerifyArgs items_from(VerifyArgs a, int first) {
 
 }  // namespace
 
-// As many lanes to an item as still give every item a place in one wave: four up
-// to 8 items a SM, two up to 16.  One launch of a block on every SM takes 3.47 ms
-// with a lane to an item, 2.77 ms with two and 2.51 ms with four (the sums shrink
-// from 2, 3, 5 and 9 products in the cyclotomic square, the line, the square and the
-// product to 1, 2, 3 and 5, or 1, 1, 2 and 3; the reductions stay).  A batch of
-// several waves whose last one would be that empty runs it as a launch of its own:
-// 4,737 items 7.0 -> 6.0 ms.
+// As many lanes to an item as still give every item a place in one wave of the SMs that
+// the launch plans with (chip_share.h): four up to 8 items a SM, two up to 16.  One
+// launch alone of a block on every SM takes 3.47 ms with a lane to an item, 2.77 ms with
+// two and 2.51 ms with four (the sums shrink from 2, 3, 5 and 9 products in the
+// cyclotomic square, the line, the square and the product to 1, 2, 3 and 5, or 1, 1, 2
+// and 3; the reductions stay).  A batch of several waves whose last one would be that
+// empty runs it as a launch of its own: 4,737 items 7.0 -> 6.0 ms.
 cudaError_t launch_verify_w(const VerifyArgs& a, const uint32_t* in_status, int sms, cudaStream_t s) {
     if (a.n <= 0) return cudaSuccess;
     cudaError_t e = configure();
     if (e != cudaSuccess) return e;
-    const int rest = a.n % (kV * sms);
-    const int split = rest == 0 ? 1 : rest <= 8 * sms ? 4 : rest <= 16 * sms ? 2 : 1;
-    const int full = split == 1 ? a.n : a.n - rest;   // items with a lane each
+    const int split = a.item_lanes ? a.item_lanes : verify_item_lanes(a.n, sms, sms);
+    const int full = split == 1 ? a.n : a.n - a.n % (kV * sms);   // items with a lane each
     if (full > 0) {
         VerifyArgs f = a;
         f.n = full;
