@@ -196,7 +196,7 @@ struct bls_ctx {
     // an identity key's table is never read (its pair is skipped), so a zero
     // c2 there does not disable the normalised path
     int normalize(const uint64_t* src, uint64_t* dst, int k, bool identity = false) {
-        CK(bls::launch_lines_normalize(src, 1, dst, d_corr + 12 * (size_t)k, d_norm_bad + k, stream));
+        CK(bls::launch_lines_normalize(src, 1, dst, d_corr + 12 * (size_t)k, d_norm_bad + k, sms, stream));
         uint8_t bad = 0;
         CK(cudaMemcpyAsync(&bad, d_norm_bad + k, 1, cudaMemcpyDeviceToHost, stream));
         CK(cudaStreamSynchronize(stream));
@@ -361,7 +361,7 @@ int ctx_init(bls_ctx* c, const bls_config* cfg) {
     uint64_t* d_q = nullptr;
     CK(cudaMalloc(&d_q, sizeof kG2Gen));
     CK(cudaMemcpyAsync(d_q, kG2Gen, sizeof kG2Gen, cudaMemcpyHostToDevice, c->stream));
-    CK(bls::launch_g2_prepare(d_q, 1, c->d_g2, c->stream));
+    CK(bls::launch_g2_prepare(d_q, 1, c->d_g2, c->sms, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     CK(cudaFree(d_q));
     return c->normalize(c->d_g2, c->d_g2_norm, 0);
@@ -419,24 +419,32 @@ class Working {
     bls_ctx* c_;
 };
 
-// lanes to an item of a verify of n items (0 where the kernel has one form only)
-int plan_lanes(bls_ctx* c, int n) {
-    return c->cfg.lanes_per_pairing == 6 && bls::six_lane_shape(c->cfg.threads_per_block) == bls::kShapeWide
-               ? c->use.plan_verify(n)
-               : 0;
+// What a verify of n items plans with: SMs for its decode, and lanes to an item (0
+// where the kernel has one form only).
+struct Plan {
+    int sms = 0, lanes = 0;
+};
+Plan plan_verify(bls_ctx* c, int n) {
+    Plan p;
+    p.sms = c->use.share(1);
+    if (c->cfg.lanes_per_pairing == 6 && bls::six_lane_shape(c->cfg.threads_per_block) == bls::kShapeWide)
+        p.lanes = c->use.plan_verify(n);
+    return p;
 }
 
 // One verify launch on the context stream.  lanes_per_pairing 1 runs the
 // thread-per-verification kernel (which decodes compressed signatures itself);
 // otherwise compressed signatures are first decoded into scratch buffers by
 // launch_g1_decompress, then the lane-parallel kernel verifies; decoded: d_xy and
-// d_st already hold them.
-int run_verify(bls_ctx* c, bls::VerifyArgs a, bool decoded = false) {
+// d_st already hold them; plan: as made already (no SMs: made here).
+int run_verify(bls_ctx* c, bls::VerifyArgs a, bool decoded = false, Plan plan = {}) {
     if (c->cfg.lanes_per_pairing == 1) {
         a.work_counter = nullptr;
         CK(bls::launch_verify(a, c->stream));
         return BLS_OK;
     }
+    if (!plan.sms) plan = plan_verify(c, a.n);
+    a.item_lanes = plan.lanes;
     const uint32_t* status = nullptr;
     if (a.sig_compressed) {
         int rc;
@@ -445,12 +453,11 @@ int run_verify(bls_ctx* c, bls::VerifyArgs a, bool decoded = false) {
             return rc;
         if (!decoded)
             CK(bls::launch_g1_decompress((const uint8_t*)a.sigs, a.n, (uint64_t*)c->d_xy.p, (int32_t*)c->d_st.p,
-                                         c->stream));
+                                         plan.sms, c->stream));
         a.sig_xy = (const uint64_t*)c->d_xy.p;
         status = (const uint32_t*)c->d_st.p;
     }
     if (a.work_counter) CK(cudaMemsetAsync(a.work_counter, 0, sizeof(int), c->stream));
-    if (!a.item_lanes) a.item_lanes = plan_lanes(c, a.n);
     CK(bls::launch_verify_lanes(a, status, c->cfg.lanes_per_pairing, c->cfg.threads_per_block, c->cfg.blocks_per_sm,
                                 c->sms, c->stream));
     return BLS_OK;
@@ -477,9 +484,9 @@ int prepare(bls_ctx* c, size_t n, int fmt, bool want_ml, bool want_gt, bool stag
 // enqueue: staged inputs -> device, verify, results -> h_res (no synchronise);
 // nhms_on_device: d_nhms was filled on the device (a hash launch) instead;
 // inputs_on_device: the caller has already queued every input copy; decoded: and the
-// launch that decodes the signatures; item_lanes: as planned already (0: planned here)
+// launch that decodes the signatures; plan: run_verify's
 int enqueue(bls_ctx* c, size_t n, int fmt, bool persistent, bool want_ml, bool want_gt,
-            bool nhms_on_device = false, bool inputs_on_device = false, bool decoded = false, int item_lanes = 0) {
+            bool nhms_on_device = false, bool inputs_on_device = false, bool decoded = false, Plan plan = {}) {
     size_t sig_bytes = n * (fmt == BLS_SIG_COMPRESSED ? 48 : 96);
     if (!inputs_on_device) {
         CK(cudaMemcpyAsync(c->d_sigs.p, c->h_sigs.p, sig_bytes, cudaMemcpyHostToDevice, c->stream));
@@ -503,8 +510,7 @@ int enqueue(bls_ctx* c, size_t n, int fmt, bool persistent, bool want_ml, bool w
     a.ml_out = want_ml ? (uint64_t*)c->d_ml.p : nullptr;
     a.gt_out = want_gt ? (uint64_t*)c->d_gt.p : nullptr;
     a.work_counter = persistent ? (int*)c->d_work.p : nullptr;
-    a.item_lanes = item_lanes;
-    int rc = run_verify(c, a, decoded);
+    int rc = run_verify(c, a, decoded, plan);
     if (rc) return rc;
     CK(cudaMemcpyAsync(c->h_res.p, a.results, n * 4, cudaMemcpyDeviceToHost, c->stream));
     return BLS_OK;
@@ -529,10 +535,11 @@ int stage_hash(bls_ctx* c, const uint8_t* msgs, const uint32_t* offsets, int n, 
         CK(bls::launch_neg_hash_decode((const uint8_t*)c->d_msg.p, (const uint32_t*)c->d_off.p, n,
                                        (const uint8_t*)c->d_dst.p, dst_len, (uint64_t*)c->d_nhms.p,
                                        (const uint8_t*)c->d_sigs.p, (uint64_t*)c->d_xy.p, (int32_t*)c->d_st.p,
-                                       c->stream));
+                                       c->use.share(1), c->stream));
     else
         CK(bls::launch_neg_hash_to_g1((const uint8_t*)c->d_msg.p, (const uint32_t*)c->d_off.p, n,
-                                      (const uint8_t*)c->d_dst.p, dst_len, (uint64_t*)c->d_nhms.p, c->stream));
+                                      (const uint8_t*)c->d_dst.p, dst_len, (uint64_t*)c->d_nhms.p,
+                                      c->use.share(1), c->stream));
     return BLS_OK;
 }
 
@@ -671,7 +678,7 @@ bool cached_table_ids(bls_ctx* c, const std::vector<const uint64_t*>& tables, st
         !ck(cudaMemsetAsync(c->d_pk_inf + first, 0, k, c->stream)) ||
         !ck(bls::launch_lines_normalize(c->d_pk + W * (size_t)first, (int)k, c->d_pk_norm + W * (size_t)first,
                                         c->d_corr + 12 * (size_t)(1 + first), c->d_norm_bad + 1 + first,
-                                        c->stream)) ||
+                                        c->use.share(1), c->stream)) ||
         !ck(cudaMemcpyAsync(bad.data(), c->d_norm_bad + 1 + first, k, cudaMemcpyDeviceToHost, c->stream)) ||
         !ck(cudaStreamSynchronize(c->stream))) {
         c->h_cached.resize(W * (size_t)first);
@@ -765,7 +772,7 @@ int bls_pk_register_affine(bls_ctx* ctx, const uint64_t* q24, int32_t* pk_id) {
     int id = ctx->n_pks;
     CK(cudaMemcpyAsync(ctx->d_in.p, q24, 24 * 8, cudaMemcpyHostToDevice, ctx->stream));
     CK(bls::launch_g2_prepare((const uint64_t*)ctx->d_in.p, 1, ctx->d_pk + (size_t)id * bls::kCoeffU64,
-                              ctx->stream));
+                              ctx->sms, ctx->stream));
     ctx->h_pk_inf[id] = 0;
     CK(cudaMemcpyAsync(ctx->d_pk_inf + id, &ctx->h_pk_inf[id], 1, cudaMemcpyHostToDevice, ctx->stream));
     int nrc = ctx->normalize(ctx->d_pk + (size_t)id * bls::kCoeffU64, ctx->d_pk_norm + (size_t)id * bls::kCoeffU64,
@@ -787,6 +794,7 @@ int bls_pk_register_affine_batch(bls_ctx* ctx, const uint64_t* q24, int n, int32
     if (n > ctx->cfg.max_pks - ctx->n_pks)
         return fail(BLS_ERR_FULL, "%d keys do not fit: %d of %d pk slots used", n, ctx->n_pks, ctx->cfg.max_pks);
     CK(cudaSetDevice(ctx->cfg.device));
+    Working call(ctx);
     const size_t k = (size_t)n;
     int rc = ctx->grow(ctx->d_in, k * 24 * 8);
     if (rc) return rc;
@@ -794,10 +802,11 @@ int bls_pk_register_affine_batch(bls_ctx* ctx, const uint64_t* q24, int n, int32
     uint64_t* tables = ctx->d_pk + (size_t)id0 * bls::kCoeffU64;
     std::vector<uint8_t> bad(k);
     CK(cudaMemcpyAsync(ctx->d_in.p, q24, k * 24 * 8, cudaMemcpyHostToDevice, ctx->stream));
-    CK(bls::launch_g2_prepare((const uint64_t*)ctx->d_in.p, n, tables, ctx->stream));
+    const int part = ctx->use.share(1);
+    CK(bls::launch_g2_prepare((const uint64_t*)ctx->d_in.p, n, tables, part, ctx->stream));
     CK(cudaMemsetAsync(ctx->d_pk_inf + id0, 0, k, ctx->stream));
     CK(bls::launch_lines_normalize(tables, n, ctx->d_pk_norm + (size_t)id0 * bls::kCoeffU64,
-                                   ctx->d_corr + 12 * (size_t)(1 + id0), ctx->d_norm_bad + 1 + id0, ctx->stream));
+                                   ctx->d_corr + 12 * (size_t)(1 + id0), ctx->d_norm_bad + 1 + id0, part, ctx->stream));
     CK(cudaMemcpyAsync(bad.data(), ctx->d_norm_bad + 1 + id0, k, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     for (size_t i = 0; i < k; ++i) {
@@ -819,6 +828,7 @@ int bls_pk_register_compressed(bls_ctx* ctx, const uint8_t* pks96, int n, int32_
     if (n > ctx->cfg.max_pks - ctx->n_pks)
         return fail(BLS_ERR_FULL, "%d keys do not fit: %d of %d pk slots used", n, ctx->n_pks, ctx->cfg.max_pks);
     CK(cudaSetDevice(ctx->cfg.device));
+    Working call(ctx);
     int rc;
     const size_t k = (size_t)n;
     if ((rc = ctx->grow(ctx->d_in, k * 96)) || (rc = ctx->grow(ctx->d_xy, k * 192)) ||
@@ -829,16 +839,17 @@ int bls_pk_register_compressed(bls_ctx* ctx, const uint8_t* pks96, int n, int32_
     std::vector<int32_t> st(k);
     std::vector<uint8_t> inf(k), bad(k);
     CK(cudaMemcpyAsync(ctx->d_in.p, pks96, k * 96, cudaMemcpyHostToDevice, ctx->stream));
+    const int part = ctx->use.share(1);
     CK(bls::launch_g2_decompress((const uint8_t*)ctx->d_in.p, n, (uint64_t*)ctx->d_xy.p, (int32_t*)ctx->d_st.p,
-                                 ctx->d_pk_inf + id0, ctx->stream));
+                                 ctx->d_pk_inf + id0, part, ctx->stream));
     CK(cudaMemcpyAsync(st.data(), ctx->d_st.p, k * 4, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     if (status) memcpy(status, st.data(), k * 4);
     for (size_t i = 0; i < k; ++i)
         if (st[i] != BLS_ST_OK) return fail(BLS_ERR_INVALID, "key %zu: decode status %d", i, st[i]);
-    CK(bls::launch_g2_prepare((const uint64_t*)ctx->d_xy.p, n, tables, ctx->stream));
+    CK(bls::launch_g2_prepare((const uint64_t*)ctx->d_xy.p, n, tables, part, ctx->stream));
     CK(bls::launch_lines_normalize(tables, n, ctx->d_pk_norm + (size_t)id0 * bls::kCoeffU64,
-                                   ctx->d_corr + 12 * (size_t)(1 + id0), ctx->d_norm_bad + 1 + id0, ctx->stream));
+                                   ctx->d_corr + 12 * (size_t)(1 + id0), ctx->d_norm_bad + 1 + id0, part, ctx->stream));
     CK(cudaMemcpyAsync(inf.data(), ctx->d_pk_inf + id0, k, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(bad.data(), ctx->d_norm_bad + 1 + id0, k, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -857,6 +868,7 @@ int bls_g2_decompress_status(bls_ctx* ctx, const uint8_t* in, int n, uint64_t* q
     if (n == 0) return BLS_OK;
     std::lock_guard<std::mutex> lk(ctx->mu);
     CK(cudaSetDevice(ctx->cfg.device));
+    Working call(ctx);
     int rc;
     const size_t k = (size_t)n;
     if ((rc = ctx->grow(ctx->d_in, k * 96)) || (rc = ctx->grow(ctx->d_xy, k * 192)) ||
@@ -864,7 +876,7 @@ int bls_g2_decompress_status(bls_ctx* ctx, const uint8_t* in, int n, uint64_t* q
         return rc;
     CK(cudaMemcpyAsync(ctx->d_in.p, in, k * 96, cudaMemcpyHostToDevice, ctx->stream));
     CK(bls::launch_g2_decompress((const uint8_t*)ctx->d_in.p, n, (uint64_t*)ctx->d_xy.p, (int32_t*)ctx->d_st.p,
-                                 nullptr, ctx->stream));
+                                 nullptr, ctx->use.share(1), ctx->stream));
     CK(cudaMemcpyAsync(q24, ctx->d_xy.p, k * 192, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(status, ctx->d_st.p, k * 4, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -957,7 +969,7 @@ int bls_verify_requests(bls_ctx* ctx, const bls_request* reqs, int nreq, int fmt
         memcpy((char*)ctx->h_nhms.p + at * 96, reqs[r].neg_hms, n * 96);
         memcpy((char*)ctx->h_pkidx.p + at * 4, reqs[r].pk_ids, n * 4);
     });
-    const int item_lanes = plan_lanes(ctx, (int)total);
+    const Plan plan = plan_verify(ctx, (int)total);
     std::vector<const void*> key = {(const void*)total, (const void*)(size_t)fmt,
                                     (const void*)(size_t)ctx->cfg.lanes_per_pairing,
                                     (const void*)(size_t)ctx->cfg.threads_per_block,
@@ -966,14 +978,16 @@ int bls_verify_requests(bls_ctx* ctx, const bls_request* reqs, int nreq, int fmt
                                     ctx->h_sigs.p, ctx->h_nhms.p, ctx->h_pkidx.p, ctx->h_res.p,
                                     // the key count the kernel checks ids against, and the table form
                                     (const void*)(size_t)ctx->n_pks, (const void*)(size_t)ctx->norm_ok,
-                                    (const void*)(size_t)item_lanes};
+                                    // the launches' forms
+                                    (const void*)(size_t)plan.lanes,
+                                    (const void*)(size_t)bls::g1_decompress_small((int)total, plan.sms)};
     if (!ctx->graph || ctx->graph_key != key) {
         ctx->drop_graph();
         if (ctx->cfg.lanes_per_pairing > 1)   // set up outside capture
             bls::verify_lanes_blocks_per_sm(ctx->cfg.lanes_per_pairing, ctx->cfg.threads_per_block);
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-        rc = enqueue(ctx, total, fmt, true, false, false, false, false, false, item_lanes);
+        rc = enqueue(ctx, total, fmt, true, false, false, false, false, false, plan);
         cudaError_t ec = cudaStreamEndCapture(ctx->stream, &g);
         if (rc) {
             if (g) cudaGraphDestroy(g);
@@ -1216,7 +1230,7 @@ int bls_verify_batch_rlc(bls_ctx* ctx, const bls_batch* b, const uint64_t* scala
     bls::RlcArgs ra{};
     if (fmt == BLS_SIG_COMPRESSED) {
         CK(bls::launch_g1_decompress((const uint8_t*)ctx->d_sigs.p, b->n, (uint64_t*)ctx->d_xy.p,
-                                     (int32_t*)ctx->d_st.p, st));
+                                     (int32_t*)ctx->d_st.p, ctx->use.share(1), st));
         ra.sig_xy = (const uint64_t*)ctx->d_xy.p;
         ra.status = (const int32_t*)ctx->d_st.p;
     } else {
@@ -1287,6 +1301,7 @@ int bls_neg_hash_to_g1(bls_ctx* ctx, const uint8_t* msgs, const uint32_t* offset
     if (n == 0) return BLS_OK;
     std::lock_guard<std::mutex> lk(ctx->mu);
     CK(cudaSetDevice(ctx->cfg.device));
+    Working call(ctx);
     if ((rc = stage_hash(ctx, msgs, offsets, n, dst, dst_len))) return rc;
     CK(cudaMemcpyAsync(out, ctx->d_nhms.p, (size_t)n * 96, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -1325,13 +1340,14 @@ int bls_g1_decompress_status(bls_ctx* ctx, const uint8_t* in, int n, uint64_t* x
     if (n == 0) return BLS_OK;
     std::lock_guard<std::mutex> lk(ctx->mu);
     CK(cudaSetDevice(ctx->cfg.device));
+    Working call(ctx);
     int rc;
     if ((rc = ctx->grow(ctx->d_in, (size_t)n * 48)) || (rc = ctx->grow(ctx->d_xy, (size_t)n * 96)) ||
         (rc = ctx->grow(ctx->d_st, (size_t)n * 4)))
         return rc;
     CK(cudaMemcpyAsync(ctx->d_in.p, in, (size_t)n * 48, cudaMemcpyHostToDevice, ctx->stream));
     CK(bls::launch_g1_decompress((const uint8_t*)ctx->d_in.p, n, (uint64_t*)ctx->d_xy.p, (int32_t*)ctx->d_st.p,
-                                 ctx->stream));
+                                 ctx->use.share(1), ctx->stream));
     CK(cudaMemcpyAsync(xy, ctx->d_xy.p, (size_t)n * 96, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(status, ctx->d_st.p, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));

@@ -151,12 +151,12 @@ __global__ void __launch_bounds__(kQuadThreads) k_neg_hash_decode(const uint8_t*
 // bls_neg_hash_to_g1 from host buffers, eight lanes against two: 1 message 0.84 and
 // 1.34 ms, 1,000 messages 0.87 and 1.37 ms, 2,368 (a warp on every scheduler) 0.88 and
 // 1.37 ms, 4,736 (two) 1.21 and 1.40 ms; 7,104 messages 1.87 against 1.42 ms.
-constexpr int kHashQuadMax = 4736;
+constexpr int kHashQuadMax = 4736;    // 32 an SM
 
 cudaError_t launch_neg_hash_to_g1(const uint8_t* msgs, const uint32_t* offsets, int n, const uint8_t* dst,
-                                  int dst_len, uint64_t* out, cudaStream_t s) {
+                                  int dst_len, uint64_t* out, int sms, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    if (n <= kHashQuadMax) {
+    if (small_batch(n, kHashQuadMax, sms)) {
         k_neg_hash_to_g1_quad<<<(unsigned)((8LL * n + kHashQuadThreads - 1) / kHashQuadThreads), kHashQuadThreads, 0, s>>>(
             msgs, offsets, n, dst, dst_len, out);
         return cudaGetLastError();
@@ -179,17 +179,17 @@ constexpr int kHashDecodeTwoMax = 2368;     // 16
 
 cudaError_t launch_neg_hash_decode(const uint8_t* msgs, const uint32_t* offsets, int n, const uint8_t* dst,
                                    int dst_len, uint64_t* out, const uint8_t* sigs, uint64_t* xy, int32_t* status,
-                                   cudaStream_t s) {
+                                   int sms, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    if (n <= kHashDecodeQuadMax) {
+    if (small_batch(n, kHashDecodeQuadMax, sms)) {
         const int hash_blocks = (8 * n + kQuadThreads - 1) / kQuadThreads;
         k_neg_hash_decode<<<hash_blocks + (n + kQuadPoints - 1) / kQuadPoints, kQuadThreads, 0, s>>>(
             msgs, offsets, n, dst, dst_len, out, hash_blocks, sigs, xy, status);
         return cudaGetLastError();
     }
-    if (n <= kHashDecodeTwoMax) {
-        const cudaError_t e = launch_neg_hash_to_g1(msgs, offsets, n, dst, dst_len, out, s);
-        return e != cudaSuccess ? e : launch_g1_decompress(sigs, n, xy, status, s);
+    if (small_batch(n, kHashDecodeTwoMax, sms)) {
+        const cudaError_t e = launch_neg_hash_to_g1(msgs, offsets, n, dst, dst_len, out, sms, s);
+        return e != cudaSuccess ? e : launch_g1_decompress(sigs, n, xy, status, sms, s);
     }
     const int hash_blocks = (n + kHashThreads / 2 - 1) / (kHashThreads / 2);
     k_neg_hash_decode_wide<<<hash_blocks + (n + kHashThreads - 1) / kHashThreads, kHashThreads, 0, s>>>(

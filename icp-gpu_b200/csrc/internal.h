@@ -78,7 +78,16 @@ struct RlcArgs {
 };
 cudaError_t launch_rlc(const RlcArgs& a, cudaStream_t s);
 cudaError_t launch_gt_product(uint64_t* gt, int n, int* counters, cudaStream_t s);
-cudaError_t launch_g1_decompress(const uint8_t* in, int n, uint64_t* xy, int32_t* status, cudaStream_t s);
+
+// The small-batch forms of the decoders, the hash and the key kernels repeat work on
+// several lanes, which loses once the SMs that a launch plans with (`sms`: ChipUse::share)
+// are full of it.  Their limits are written down for the chip they were measured on.
+constexpr int kMeasuredSms = 148;
+inline bool small_batch(int n, int limit, int sms) { return (int64_t)n * kMeasuredSms <= (int64_t)limit * sms; }
+
+cudaError_t launch_g1_decompress(const uint8_t* in, int n, uint64_t* xy, int32_t* status, int sms, cudaStream_t s);
+// whether that launch takes the small-batch form
+bool g1_decompress_small(int n, int sms);
 // the same decode in whole-SM blocks, at most max_sms of them (grid-stride):
 // the serving ring's decoder, which must stay within the SMs left to it;
 // check_subgroup false leaves the subgroup test to launch_g1_subgroup_sms
@@ -89,17 +98,17 @@ cudaError_t launch_g1_decompress_sms(const uint8_t* in, int n, uint64_t* xy, int
 cudaError_t launch_g1_subgroup_sms(const uint64_t* xy, const int32_t* status, int n, int32_t* sub, int max_sms,
                                    cudaStream_t s);
 cudaError_t launch_neg_hash_to_g1(const uint8_t* msgs, const uint32_t* offsets, int n, const uint8_t* dst,
-                                  int dst_len, uint64_t* out, cudaStream_t s);
+                                  int dst_len, uint64_t* out, int sms, cudaStream_t s);
 // launch_neg_hash_to_g1 of n messages and launch_g1_decompress of n signatures
 cudaError_t launch_neg_hash_decode(const uint8_t* msgs, const uint32_t* offsets, int n, const uint8_t* dst,
                                    int dst_len, uint64_t* out, const uint8_t* sigs, uint64_t* xy, int32_t* status,
-                                   cudaStream_t s);
-cudaError_t launch_g2_decompress(const uint8_t* in, int n, uint64_t* q, int32_t* status, uint8_t* identity,
+                                   int sms, cudaStream_t s);
+cudaError_t launch_g2_decompress(const uint8_t* in, int n, uint64_t* q, int32_t* status, uint8_t* identity, int sms,
                                  cudaStream_t s);
-cudaError_t launch_g2_prepare(const uint64_t* q, int n, uint64_t* out, cudaStream_t s);
+cudaError_t launch_g2_prepare(const uint64_t* q, int n, uint64_t* out, int sms, cudaStream_t s);
 // n line tables divided row by row by their c2, with each table's Miller
 // correction factor (12 u64) and a flag set when a c2 is zero (table copied)
-cudaError_t launch_lines_normalize(const uint64_t* raw, int n, uint64_t* norm, uint64_t* corr, uint8_t* bad,
+cudaError_t launch_lines_normalize(const uint64_t* raw, int n, uint64_t* norm, uint64_t* corr, uint8_t* bad, int sms,
                                    cudaStream_t s);
 // Block shapes of the six-lane (Fp2-lane) kernels, by threads per block:
 // kShapeFive (64 threads, two warps, five items per block: k_verify_fp2) and

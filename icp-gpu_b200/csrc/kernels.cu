@@ -303,12 +303,12 @@ __global__ void __launch_bounds__(64) k_lines_normalize_table(const uint64_t* ra
 // (least work: the whole set in one wave, where the row form would square each
 // row's c2 separately and take many waves).  With the line tables themselves: 2,368
 // keys 2.11 against 2.53 ms, 4,736 keys 3.80 against 2.80 ms.
-constexpr int kRowsMaxTables = 2960;
+constexpr int kRowsMaxTables = 2960;    // 20 an SM
 
-cudaError_t launch_lines_normalize(const uint64_t* raw, int n, uint64_t* norm, uint64_t* corr, uint8_t* bad,
+cudaError_t launch_lines_normalize(const uint64_t* raw, int n, uint64_t* norm, uint64_t* corr, uint8_t* bad, int sms,
                                    cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    if (n <= kRowsMaxTables)
+    if (small_batch(n, kRowsMaxTables, sms))
         k_lines_normalize_rows<<<n, kNormThreads, 0, s>>>(raw, n, norm, corr, bad);
     else
         k_lines_normalize_table<<<(n + 63) / 64, 64, 0, s>>>(raw, n, norm, corr, bad);
@@ -328,9 +328,11 @@ cudaError_t launch_verify(const VerifyArgs& a, cudaStream_t s) {
 // SM) 1.36 against 1.83 ms, 14,208 points 2.20 against 1.88 ms.
 constexpr int kQuadMaxPoints = 9472;
 
-cudaError_t launch_g1_decompress(const uint8_t* in, int n, uint64_t* xy, int32_t* status, cudaStream_t s) {
+bool g1_decompress_small(int n, int sms) { return small_batch(n, kQuadMaxPoints, sms); }
+
+cudaError_t launch_g1_decompress(const uint8_t* in, int n, uint64_t* xy, int32_t* status, int sms, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    if (n <= kQuadMaxPoints)
+    if (g1_decompress_small(n, sms))
         k_g1_decompress_quad<<<(n + kQuadPoints - 1) / kQuadPoints, kQuadThreads, 0, s>>>(in, n, xy, status);
     else
         k_g1_decompress<<<(n + 127) / 128, 128, 0, s>>>(in, n, xy, status);
@@ -368,21 +370,21 @@ cudaError_t launch_g1_subgroup_sms(const uint64_t* xy, const int32_t* status, in
 // 1.35 and 2.30 ms, 2,368 keys (a warp on every scheduler) 1.43 and 2.37 ms, 4,736
 // keys 2.11 and 2.46 ms, 9,472 keys 4.09 and 2.61 ms; bls_pk_register_affine_batch of
 // 500 keys 0.96 and 2.59 ms, 4,736 keys 2.80 and 4.20 ms, 9,472 keys 3.71 and 4.30 ms.
-constexpr int kOctMaxKeys = 4736;
+constexpr int kOctMaxKeys = 4736;    // 32 an SM
 
-cudaError_t launch_g2_decompress(const uint8_t* in, int n, uint64_t* q, int32_t* status, uint8_t* identity,
+cudaError_t launch_g2_decompress(const uint8_t* in, int n, uint64_t* q, int32_t* status, uint8_t* identity, int sms,
                                  cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    if (n <= kOctMaxKeys)
+    if (small_batch(n, kOctMaxKeys, sms))
         k_g2_decompress_oct<<<(8 * n + kOctThreads - 1) / kOctThreads, kOctThreads, 0, s>>>(in, n, q, status, identity);
     else
         k_g2_decompress<<<(n + 63) / 64, 64, 0, s>>>(in, n, q, status, identity);
     return cudaGetLastError();
 }
 
-cudaError_t launch_g2_prepare(const uint64_t* q, int n, uint64_t* out, cudaStream_t s) {
+cudaError_t launch_g2_prepare(const uint64_t* q, int n, uint64_t* out, int sms, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    if (n <= kOctMaxKeys)
+    if (small_batch(n, kOctMaxKeys, sms))
         k_g2_prepare_oct<<<(8 * n + kOctThreads - 1) / kOctThreads, kOctThreads, 0, s>>>(q, n, out);
     else
         k_g2_prepare<<<(n + 63) / 64, 64, 0, s>>>(q, n, out);

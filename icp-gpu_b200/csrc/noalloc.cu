@@ -88,6 +88,11 @@ __global__ void k_check_key_index(const int32_t* __restrict__ pk_index, int n, i
     idx[i] = ok ? k : 0;
     if (!ok && status[i] == BLS_ST_OK) status[i] = BLS_ST_BAD_KEY_INDEX;
 }
+cudaError_t launch_check_key_index(const int32_t* pk_index, int n, int n_tables, int32_t* idx, int32_t* status,
+                                   cudaStream_t s) {
+    k_check_key_index<<<(n + 255) / 256, 256, 0, s>>>(pk_index, n, n_tables, idx, status);
+    return cudaGetLastError();
+}
 
 }  // namespace
 }  // namespace bls
@@ -115,10 +120,10 @@ extern "C" int bls_verify_compressed_noalloc(const uint8_t* sigs48, const uint64
     int32_t* status = reinterpret_cast<int32_t*>(base + bls::kXyBytes);
     int32_t* idx = reinterpret_cast<int32_t*>(base + bls::kXyBytes + bls::kStatusBytes);
     int* counter = reinterpret_cast<int*>(base + bls::kXyBytes + bls::kStatusBytes + bls::kIndexBytes);
-    if (cudaMemsetAsync(counter, 0, sizeof(int), s) != cudaSuccess) return BLS_ERR_CUDA;
-    if (bls::launch_g1_decompress(sigs48, n, xy, status, s) != cudaSuccess) return BLS_ERR_CUDA;
-    bls::k_check_key_index<<<(n + 255) / 256, 256, 0, s>>>(pk_index, n, n_tables, idx, status);
-    if (cudaGetLastError() != cudaSuccess) return BLS_ERR_CUDA;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) return BLS_ERR_CUDA;
+    std::lock_guard<std::mutex> lk(d.mu);
+    d.use.begin(dev, sms);
     bls::VerifyArgs a{};
     a.sigs = sigs48;
     a.sig_compressed = 1;
@@ -131,17 +136,17 @@ extern "C" int bls_verify_compressed_noalloc(const uint8_t* sigs48, const uint64
     a.n = n;
     a.results = results;
     a.work_counter = counter;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) return BLS_ERR_CUDA;
-    std::lock_guard<std::mutex> lk(d.mu);
-    d.use.begin(dev, sms);
-    if (lanes_per_pairing == 6) a.item_lanes = d.use.plan_verify(n);
-    const bool ok = bls::launch_verify_lanes(a, reinterpret_cast<const uint32_t*>(status), lanes_per_pairing, 0, 0, sms,
-                                             s) == cudaSuccess;
+    const int part = d.use.share(1);
+    const bool ok = cudaMemsetAsync(counter, 0, sizeof(int), s) == cudaSuccess &&
+                    bls::launch_g1_decompress(sigs48, n, xy, status, part, s) == cudaSuccess &&
+                    bls::launch_check_key_index(pk_index, n, n_tables, idx, status, s) == cudaSuccess;
+    if (ok && lanes_per_pairing == 6) a.item_lanes = d.use.plan_verify(n);
+    const bool done = ok && bls::launch_verify_lanes(a, reinterpret_cast<const uint32_t*>(status), lanes_per_pairing, 0,
+                                                     0, sms, s) == cudaSuccess;
     // a captured call runs nothing yet
-    if (ok && capture == cudaStreamCaptureStatusNone && cudaEventRecord(d.ran, s) == cudaSuccess)
+    if (done && capture == cudaStreamCaptureStatusNone && cudaEventRecord(d.ran, s) == cudaSuccess)
         d.use.end_when(bls::event_done, d.ran);
     else
         d.use.end();
-    return ok ? BLS_OK : BLS_ERR_CUDA;
+    return done ? BLS_OK : BLS_ERR_CUDA;
 }

@@ -199,7 +199,8 @@ struct bls_server {
         a.work_counter = (int*)s.d_work;
         const uint32_t* status = nullptr;
         if (a.sig_compressed) {
-            if (bls::launch_g1_decompress((const uint8_t*)s.d_sigs, a.n, (uint64_t*)s.d_xy, (int32_t*)s.d_st, st))
+            if (bls::launch_g1_decompress((const uint8_t*)s.d_sigs, a.n, (uint64_t*)s.d_xy, (int32_t*)s.d_st,
+                                          s.use.share(1, false), st))
                 return BLS_ERR_CUDA;
             a.sig_xy = (const uint64_t*)s.d_xy;
             status = (const uint32_t*)s.d_st;
@@ -294,7 +295,7 @@ struct bls_server {
                                                        ring.d_sigs + 12 * (size_t)from, ring.d_st + from,
                                                        kDecSmsPerRound, !ring.split, st)
                        : bls::launch_g1_decompress(ring.d_comp + 48 * (size_t)from, (int)count,
-                                                   ring.d_sigs + 12 * (size_t)from, ring.d_st + from, st);
+                                                   ring.d_sigs + 12 * (size_t)from, ring.d_st + from, view.sms, st);
         };
         if (decode(s0, first) || (first < n && decode(0, n - first))) return BLS_ERR_CUDA;
         return BLS_OK;
