@@ -47,7 +47,7 @@ class Resident:
         self.ctx.sync()
         assert (self.res.cpu().numpy() == self.want).all()
         self.res.zero_()
-        torch.cuda.synchronize()
+        torch.cuda.current_stream().synchronize()
 
 
 def seconds(resident, repeats=8):
@@ -80,9 +80,11 @@ def test_launches_side_by_side(wl, sms):
 
 
 def test_threads_with_a_context_each(wl, sms):
-    """uneven batches, host and device entry points, a capture and a server beside them"""
+    """uneven batches, host and device entry points, and beside them a server and a
+    context that captures its launches"""
     sizes = [1, 200, 8 * sms, 16 * sms + 5, 32 * sms + 9]
     res = [Resident(wl, n, seed=10 + n) for n in sizes]
+    captured = Resident(wl, 8 * sms, seed=9)
     errors = []
 
     def work(r):
@@ -110,10 +112,9 @@ def test_threads_with_a_context_each(wl, sms):
 
     def capture():
         try:
-            r = res[2]
             for _ in range(6):
-                got = r.ctx.verify_requests([r.host], compressed=True)
-                assert (np.concatenate(got) == r.want).all()
+                got = captured.ctx.verify_requests([captured.host], compressed=True)
+                assert (np.concatenate(got) == captured.want).all()
         except BaseException as e:     # noqa: BLE001
             errors.append(e)
 
@@ -123,7 +124,7 @@ def test_threads_with_a_context_each(wl, sms):
         t.start()
     for t in threads:
         t.join()
-    for r in res:
+    for r in res + [captured]:
         r.ctx.close()
     if errors:
         raise errors[0]
