@@ -1090,6 +1090,103 @@ def encode_pair(c, h):
     return w + [(co & 15) | (r << 8) for co, r in c.lins[h]]
 
 
+# ---------------------------------------------------------------- meetings of the 32-item kernel
+# After an op the block's warps meet before the next one; two kinds of op need less.
+# From one cyclotomic square to the next the coefficients fall into sets that do not
+# read each other, and each set meets by itself (so one may be many squares ahead).  A
+# line load reads no Fp12 value and leaves no partial sum, so between a square and a
+# line load nobody waits.  meeting_kinds says which meeting follows each op, and
+# check_meetings proves that it is enough.
+MEET_ALL, MEET_SETS, MEET_NONE = range(3)
+MEET_SHIFT = 23     # of the kind in an op's word
+
+
+def cyc_sets(outs=None):
+    """the sets of coefficients of the cyclotomic square whose outputs read none of another set's"""
+    if outs is None:
+        outs = dict((n, o) for n, o, _ in build())["CYCSQR"]
+    of = list(range(6))
+    for k, o in enumerate(outs):
+        for r in [r for t in o.terms for r in (t.x, t.y) if r is not None] + [r for _, r in o.lins] + [o.dst]:
+            if r >> 4 != B_K:
+                a, b = of[k], of[r & 15]
+                of = [a if v == b else v for v in of]
+    return [{k for k in range(6) if of[k] == v} for v in sorted(set(of))]
+
+
+def kernel_ops(seq):
+    """the sequence as verify_w.cu runs it: a line load takes the LSCALE behind it along"""
+    lscale = [n for n, _, _ in PROGRAMS].index("LSCALE")
+    return [op for op in seq if op[0] != lscale]
+
+
+def meeting_kinds(ops):
+    """the meeting after each op of kernel_ops(seq), by it and the next one"""
+    names = [n for n, _, _ in PROGRAMS]
+    kinds = []
+    for op, nxt in zip(ops, ops[1:] + [None]):
+        pair = (op[0], nxt[0] if nxt else None)
+        kinds.append(MEET_SETS if pair == (names.index("CYCSQR"),) * 2 else
+                     MEET_NONE if pair == (names.index("SQR"), OP_LOAD_LINES) else MEET_ALL)
+    return kinds
+
+
+def warp_accesses(op, progs):
+    """per coefficient k, what its two warps touch in shared memory: (slots read, slots
+    written, partial-sum slots), slots as in op_slots"""
+    code, d, a, b, _ = op
+    code &= ~COND_ML
+    base = {B_D: ("g", 6 * d), B_A: ("g", 6 * a), B_B: ("g", 6 * b), B_C: ("c", 0), B_K: ("k", 0),
+            B_T: ("g", 6 * T_GROUP)}
+
+    def at(r):
+        sp, off = base[r >> 4]
+        return sp, off + (r & 15)
+    res = []
+    for k in range(6):
+        c = line_pair(k) if code == OP_LOAD_LINES else progs[code][k]
+        rd, wr, parts = set(), set(), set()
+        if code == OP_LOAD_LINES and c is None:
+            wr.add(("c", 6 * (k // 3) + k % 3))                    # c2, stored as it is
+        if c is not None:
+            wr.add(at(c.dst))
+            for h in range(2):
+                for uf, ur, _, vr, store in c.prods[h]:
+                    rd |= {at(vr)} if uf == X_LINE else {at(ur), at(vr)}
+                    if store:
+                        parts.add(store[1])
+                parts |= {sl for sl, _ in c.adds[h]}
+                rd |= {at(r) for _, r in c.lins[h]}
+        res.append((rd, wr, parts))
+    return res
+
+
+def check_meetings(ops, kinds, sets, progs=None):
+    """assert that no two warps that `kinds` leaves unordered touch a word of which one
+    writes, whether the ops of the Miller value run or not"""
+    progs = progs or [pairs(outs) for _, outs, _ in build()]
+    touched = {op: warp_accesses(op, progs) for op in set(ops)
+               if op[0] & ~COND_ML < len(PROGRAMS) or op[0] == OP_LOAD_LINES}
+    for ml in (True, False):
+        run = [i for i, op in enumerate(ops) if ml or not op[0] & COND_ML]
+        for at, i in enumerate(run):
+            same = False                      # a meeting of the sets lies between
+            for prev, j in zip(run[at:], run[at + 1:]):
+                if kinds[prev] == MEET_ALL:
+                    break
+                assert ops[i] in touched and ops[j] in touched, "only programs and line loads go without a meeting"
+                same = same or kinds[prev] == MEET_SETS
+                if same and kinds[prev] == MEET_NONE:
+                    raise AssertionError("a meeting left out within a run of cyclotomic squares")
+                one, two = touched[ops[i]], touched[ops[j]]
+                for k in range(6):
+                    for l in range(6):
+                        if same and any(k in s and l in s for s in sets):
+                            continue
+                        (r0, w0, p0), (r1, w1, p1) = one[k], two[l]
+                        assert not (w0 & (r1 | w1)) and not (r0 & w1) and not (p0 & p1), (ops[i], ops[j], k, l)
+
+
 # operand pairs with a case of their own in the kernel (kComboGeneric: by form)
 COMBOS = [(X_S, X_0), (X_N1, X_S), (X_0, X_D10), (X_2X0, X_1), (X_S, X_D01), (X_D01, X_S), (X_2X0, X_N1), (X_2X1, X_0),
           (X_S, X_2X0), (X_2N1, X_S), (X_2X0, X_D10), (X_D01, X_2S), (X_2X0, X_2N1), (X_2X1, X_2X0)]
@@ -1274,6 +1371,16 @@ def emit(path):
                    for i, op in enumerate(seq[:-1]))
     for seq in seqs:   # verify_w.cu stores a program's outputs without a barrier after its reads
         assert all(no_war(op) for op in seq if (op[0] & ~COND_ML) < len(PROGRAMS))
+    sets = cyc_sets()
+    assert len(sets) == 2
+    for seq in seqs:
+        check_meetings(kernel_ops(seq), meeting_kinds(kernel_ops(seq)), sets)
+    L.append("// which warps of the 32-item kernel meet after an op (bits kMeetShift and up of its word): the")
+    L.append("// block's; the coefficients in kMeetSet and the others, each among themselves; none")
+    L.append("constexpr uint32_t kMeetAll = %d, kMeetSets = %d, kMeetNone = %d, kMeetShift = %d;"
+             % (MEET_ALL, MEET_SETS, MEET_NONE, MEET_SHIFT))
+    L.append("constexpr uint32_t kMeetSet = 0x%xu;" % sum(1 << k for k in sets[0]))
+    L.append("constexpr int kMeetSetSize = %d;" % len(sets[0]))
     L.append("// Fp12 groups the sequences touch (operands, results, the inverse's temporaries)")
     L.append("constexpr int kGroupsUsed = %d;" % groups_used(seqs))
     L.append("// the group that holds Gt at the end of each sequence (raw, normalised)")
@@ -1282,7 +1389,9 @@ def emit(path):
     L.append("constexpr int kSeqLenRaw = %d, kSeqLenNorm = %d;" % (len(seqs[0]), len(seqs[1])))
     L.append("__device__ __constant__ uint32_t kSeq[2][%d] = {" % n)
     for seq in seqs:
-        words = [encode_op(op) for op in seq] + [0] * (n - len(seq))
+        kinds = iter(meeting_kinds(kernel_ops(seq)))
+        words = [encode_op(op) | (next(kinds) << MEET_SHIFT if op in kernel_ops([op]) else 0) for op in seq]
+        words += [0] * (n - len(seq))
         L.append("  {")
         for i in range(0, len(words), 8):
             L.append("    " + ", ".join("0x%05xu" % w for w in words[i:i + 8]) + ",")

@@ -392,17 +392,15 @@ __device__ __forceinline__ void run(int pid, const Sm& s, int k, int half, const
     }
 }
 
-// The meeting after a program, before the op `next` (a code): the whole block's,
-// but for two cases in which fewer warps, or none, have anything to wait for.
-// From one cyclotomic square to the next (groups A and D change places) the
-// values fall into two sets that do not read each other: coefficients 0 and 4, and
-// the rest.  And a line load after a square reads no Fp12 value and writes line
-// slots that were last read before the square.
-__device__ __forceinline__ void meet(uint32_t code, uint32_t next, int k) {
-    if (code == (uint32_t)f2::P_CYCSQR && next == (uint32_t)f2::P_CYCSQR) {
-        if (k == 0 || k == 4) asm volatile("bar.sync 7, 128;" ::: "memory");
-        else asm volatile("bar.sync 8, 256;" ::: "memory");
-    } else if (!(code == (uint32_t)f2::P_SQR && next == f2::kOpLoadLines)) {
+// The meeting after the op `e`: the block's warps, or, where the generator has proved
+// that they touch nothing of each other's (gen_fp2ops.py: check_meetings), only those of
+// a set of coefficients, or none.
+__device__ __forceinline__ void meet(uint32_t e, int k) {
+    const uint32_t kind = (e >> f2::kMeetShift) & 3u;
+    if (kind == f2::kMeetSets) {
+        if ((f2::kMeetSet >> k) & 1u) asm volatile("bar.sync 7, %0;" ::"n"(64 * f2::kMeetSetSize) : "memory");
+        else asm volatile("bar.sync 8, %0;" ::"n"(64 * (6 - f2::kMeetSetSize)) : "memory");
+    } else if (kind == f2::kMeetAll) {
         __syncthreads();
     }
 }
@@ -660,7 +658,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_verify_w(VerifyArgs a, const ui
             }
             if (code < (uint32_t)f2::kNumPrograms || code == f2::kOpLoadLines) {
                 run<kSplit>(pid, s, k, half, bs, line);
-                meet(code, st + 1 < seq_len ? f2::kSeq[norm][st + 1] & 31u : 0u, k);
+                meet(e, k);
             } else if (code == f2::kOpLoadCorr) {
                 // the generator's and the key's Miller correction factors into the c2 slots
                 if (k < 2) {
