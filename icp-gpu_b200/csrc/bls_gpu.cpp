@@ -419,6 +419,18 @@ class Working {
     bls_ctx* c_;
 };
 
+// Held by a call that queues copies from or to its caller's memory: whichever way it
+// returns, nothing queued still uses that memory (page-locked buffers are read and
+// written by the copies themselves).
+class Settled {
+  public:
+    explicit Settled(bls_ctx* c) : c_(c) {}
+    ~Settled() { cudaStreamSynchronize(c_->stream); }
+
+  private:
+    bls_ctx* c_;
+};
+
 // What a verify of n items plans with: SMs for its decode, and lanes to an item (0
 // where the kernel has one form only).
 struct Plan {
@@ -516,13 +528,10 @@ int enqueue(bls_ctx* c, size_t n, int fmt, bool persistent, bool want_ml, bool w
     return BLS_OK;
 }
 
-// messages + offsets + domain to the device, then -H(m_i) into d_nhms; decode: and
+// messages + offsets (check_offsets) + domain to the device, then -H(m_i) into d_nhms; decode: and
 // the n signatures of d_sigs into d_xy and d_st (grown by prepare)
 int stage_hash(bls_ctx* c, const uint8_t* msgs, const uint32_t* offsets, int n, const uint8_t* dst, int dst_len,
                bool decode = false) {
-    if (offsets[0] != 0) return fail(BLS_ERR_INVALID, "offsets[0] must be 0");
-    for (int i = 0; i < n; ++i)
-        if (offsets[i + 1] < offsets[i]) return fail(BLS_ERR_INVALID, "offsets decrease at %d", i);
     const size_t bytes = offsets[n];
     int rc;
     if ((rc = c->grow(c->d_msg, bytes ? bytes : 1)) || (rc = c->grow(c->d_off, ((size_t)n + 1) * 4)) ||
@@ -548,6 +557,13 @@ int check_hash_args(const uint8_t* msgs, const uint32_t* offsets, int n, const u
     if (!offsets || (dst_len > 0 && !dst)) return fail(BLS_ERR_INVALID, "NULL argument");
     if (dst_len < 0 || dst_len > 255) return fail(BLS_ERR_INVALID, "dst_len %d outside 0..255", dst_len);
     if (n > 0 && offsets[n] > 0 && !msgs) return fail(BLS_ERR_INVALID, "msgs is NULL");
+    return BLS_OK;
+}
+
+int check_offsets(const uint32_t* offsets, int n) {
+    if (offsets[0] != 0) return fail(BLS_ERR_INVALID, "offsets[0] must be 0");
+    for (int i = 0; i < n; ++i)
+        if (offsets[i + 1] < offsets[i]) return fail(BLS_ERR_INVALID, "offsets decrease at %d", i);
     return BLS_OK;
 }
 
@@ -748,6 +764,7 @@ int bls_pk_register_coeffs(bls_ctx* ctx, const uint64_t* coeffs, int is_identity
     std::lock_guard<std::mutex> lk(ctx->mu);
     if (ctx->n_pks >= ctx->cfg.max_pks) return fail(BLS_ERR_FULL, "all %d pk slots used", ctx->cfg.max_pks);
     CK(cudaSetDevice(ctx->cfg.device));
+    Settled copies(ctx);
     int id = ctx->n_pks;
     CK(cudaMemcpyAsync(ctx->d_pk + (size_t)id * bls::kCoeffU64, coeffs, bls::kCoeffU64 * 8,
                        cudaMemcpyHostToDevice, ctx->stream));
@@ -767,6 +784,7 @@ int bls_pk_register_affine(bls_ctx* ctx, const uint64_t* q24, int32_t* pk_id) {
     std::lock_guard<std::mutex> lk(ctx->mu);
     if (ctx->n_pks >= ctx->cfg.max_pks) return fail(BLS_ERR_FULL, "all %d pk slots used", ctx->cfg.max_pks);
     CK(cudaSetDevice(ctx->cfg.device));
+    Settled copies(ctx);
     int rc = ctx->grow(ctx->d_in, 24 * 8);
     if (rc) return rc;
     int id = ctx->n_pks;
@@ -794,6 +812,7 @@ int bls_pk_register_affine_batch(bls_ctx* ctx, const uint64_t* q24, int n, int32
     if (n > ctx->cfg.max_pks - ctx->n_pks)
         return fail(BLS_ERR_FULL, "%d keys do not fit: %d of %d pk slots used", n, ctx->n_pks, ctx->cfg.max_pks);
     CK(cudaSetDevice(ctx->cfg.device));
+    Settled copies(ctx);
     Working call(ctx);
     const size_t k = (size_t)n;
     int rc = ctx->grow(ctx->d_in, k * 24 * 8);
@@ -828,6 +847,7 @@ int bls_pk_register_compressed(bls_ctx* ctx, const uint8_t* pks96, int n, int32_
     if (n > ctx->cfg.max_pks - ctx->n_pks)
         return fail(BLS_ERR_FULL, "%d keys do not fit: %d of %d pk slots used", n, ctx->n_pks, ctx->cfg.max_pks);
     CK(cudaSetDevice(ctx->cfg.device));
+    Settled copies(ctx);
     Working call(ctx);
     int rc;
     const size_t k = (size_t)n;
@@ -868,6 +888,7 @@ int bls_g2_decompress_status(bls_ctx* ctx, const uint8_t* in, int n, uint64_t* q
     if (n == 0) return BLS_OK;
     std::lock_guard<std::mutex> lk(ctx->mu);
     CK(cudaSetDevice(ctx->cfg.device));
+    Settled copies(ctx);
     Working call(ctx);
     int rc;
     const size_t k = (size_t)n;
@@ -888,6 +909,7 @@ int bls_pk_table(bls_ctx* ctx, int32_t pk_id, uint64_t* coeffs) {
     std::lock_guard<std::mutex> lk(ctx->mu);
     if (pk_id < -1 || pk_id >= ctx->n_pks) return fail(BLS_ERR_INVALID, "unknown pk id %d", pk_id);
     CK(cudaSetDevice(ctx->cfg.device));
+    Settled copies(ctx);
     const uint64_t* src = pk_id < 0 ? ctx->d_g2 : ctx->d_pk + (size_t)pk_id * bls::kCoeffU64;
     CK(cudaMemcpyAsync(coeffs, src, bls::kCoeffU64 * 8, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -905,6 +927,7 @@ int bls_verify_batch(bls_ctx* ctx, const bls_batch* b, int32_t* results) {
     int rc;
     if ((rc = check_ids(ctx, b->pk_ids, b->n))) return rc;
     CK(cudaSetDevice(ctx->cfg.device));
+    Settled copies(ctx);
     Working call(ctx);
     size_t n = (size_t)b->n;
     size_t sig_bytes = n * (b->sig_format == BLS_SIG_COMPRESSED ? 48 : 96);
@@ -943,6 +966,7 @@ int bls_verify_requests(bls_ctx* ctx, const bls_request* reqs, int nreq, int fmt
     for (int r = 0; r < nreq; ++r)
         if ((rc = check_ids(ctx, reqs[r].pk_ids, reqs[r].n))) return rc;
     CK(cudaSetDevice(ctx->cfg.device));
+    Settled copies(ctx);
     Working call(ctx);
     const size_t sb = fmt == BLS_SIG_COMPRESSED ? 48 : 96;
     if (mode == BLS_MODE_PLAIN) {
@@ -1185,6 +1209,7 @@ int bls_verify_batch_rlc(bls_ctx* ctx, const bls_batch* b, const uint64_t* scala
     int rc;
     if ((rc = check_ids(ctx, b->pk_ids, b->n))) return rc;
     CK(cudaSetDevice(ctx->cfg.device));
+    Settled copies(ctx);
     Working call(ctx);
     // items grouped by key; key slots in increasing id; tiles of one key
     std::vector<int32_t> start(ctx->n_pks + 1, 0), order(n), keys, key_tile, tiles;
@@ -1299,8 +1324,10 @@ int bls_neg_hash_to_g1(bls_ctx* ctx, const uint8_t* msgs, const uint32_t* offset
     int rc;
     if ((rc = check_hash_args(msgs, offsets, n, dst, dst_len))) return rc;
     if (n == 0) return BLS_OK;
+    if ((rc = check_offsets(offsets, n))) return rc;
     std::lock_guard<std::mutex> lk(ctx->mu);
     CK(cudaSetDevice(ctx->cfg.device));
+    Settled copies(ctx);
     Working call(ctx);
     if ((rc = stage_hash(ctx, msgs, offsets, n, dst, dst_len))) return rc;
     CK(cudaMemcpyAsync(out, ctx->d_nhms.p, (size_t)n * 96, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1317,8 +1344,9 @@ int bls_verify_messages(bls_ctx* ctx, int fmt, const void* sigs, const uint8_t* 
     if (!sigs || !pk_ids) return fail(BLS_ERR_INVALID, "NULL input array");
     if (fmt != BLS_SIG_AFFINE && fmt != BLS_SIG_COMPRESSED) return fail(BLS_ERR_INVALID, "unknown sig_format %d", fmt);
     std::lock_guard<std::mutex> lk(ctx->mu);
-    if ((rc = check_ids(ctx, pk_ids, n))) return rc;
+    if ((rc = check_ids(ctx, pk_ids, n)) || (rc = check_offsets(offsets, n))) return rc;
     CK(cudaSetDevice(ctx->cfg.device));
+    Settled copies(ctx);
     Working call(ctx);
     const size_t k = (size_t)n;
     if ((rc = prepare(ctx, k, fmt, false, false, false))) return rc;
@@ -1340,6 +1368,7 @@ int bls_g1_decompress_status(bls_ctx* ctx, const uint8_t* in, int n, uint64_t* x
     if (n == 0) return BLS_OK;
     std::lock_guard<std::mutex> lk(ctx->mu);
     CK(cudaSetDevice(ctx->cfg.device));
+    Settled copies(ctx);
     Working call(ctx);
     int rc;
     if ((rc = ctx->grow(ctx->d_in, (size_t)n * 48)) || (rc = ctx->grow(ctx->d_xy, (size_t)n * 96)) ||
@@ -1466,6 +1495,7 @@ int gpu_batch_bls_verify(const uint64_t* sigs, const uint64_t* neg_hms, const ui
     std::lock_guard<std::mutex> lk(c->mu);
     auto body = [&]() -> int {
         CK(cudaSetDevice(c->cfg.device));
+        Settled copies(c);
         Working call(c);
         size_t n = (size_t)M;
         const size_t W = bls::kCoeffU64;
