@@ -166,3 +166,30 @@ def test_small_batch_forms_side_by_side(sms):
     finally:
         for c in ctxs:
             c.close()
+
+
+def test_captures_beside_running_work(wl, sms):
+    """a capture (of the strict kind, which a plain event query would end) of the device
+    entry point while another context's work runs, replayed twice"""
+    other, own = Resident(wl, 32 * sms, seed=1), Resident(wl, 300, seed=2)
+    for r in (other, own):
+        r.launch()
+        r.check()                                   # buffers grown
+    stream = torch.cuda.ExternalStream(own.ctx.stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        graph.capture_begin(capture_error_mode="global")
+        for _ in range(3):
+            other.launch()
+        own.launch()
+        graph.capture_end()
+    other.check()
+    for _ in range(2):
+        with torch.cuda.stream(stream):
+            graph.replay()
+        own.check()
+    own.launch()
+    own.check()
+    del graph
+    other.ctx.close()
+    own.ctx.close()
