@@ -41,16 +41,18 @@ N_KEYS = 40
 SEED = 2
 METRIC = "BLS12-381 verifies/s, batched vs plain launch, bit-exact; serve p50/p99 ms"
 
-# Multiplies per verification of the generated op sequence in its half-coefficient
-# form (the five-item kernel's; counted by gen_fp2ops.py over the 646 programs of
-# one verification): 20,684 products of 12 x 12 limbs, each by one level of limb
-# Karatsuba (three 6 x 6 products: 108 pairs of mul.lo and mul.hi, 216 multiplies),
-# and 7,284 Montgomery reductions (12 rows of 12 pairs and one mul.lo, 300) =
-# 6,652,944.  The twelve-warp kernel's paired-warp form of the same programs has
-# 19,868 products.
+# 12 x 12-limb products and Montgomery reductions per verification, counted from the
+# generated op sequence: a product is one level of limb Karatsuba (three 6 x 6
+# products: 108 pairs of mul.lo and mul.hi, 216 multiplies), a reduction 12 rows of 12
+# pairs and one mul.lo (300).  The five-item kernel (k_verify_fp2) runs the
+# half-coefficient form of the programs, the 32-item kernel (k_verify_w) the paired-warp
+# form.
 OWN_PRODUCTS_PER_VERIFY = 20684
 OWN_REDC_PER_VERIFY = 7284
-IMAD_PER_VERIFY = OWN_PRODUCTS_PER_VERIFY * 216 + OWN_REDC_PER_VERIFY * 300
+PAIRED_PRODUCTS_PER_VERIFY = 19868
+PAIRED_REDC_PER_VERIFY = 7283
+OWN_WORK = {"k_verify_fp2": (OWN_PRODUCTS_PER_VERIFY, OWN_REDC_PER_VERIFY),
+            "k_verify_w": (PAIRED_PRODUCTS_PER_VERIFY, PAIRED_REDC_PER_VERIFY)}
 IMAD_PER_CLK_PER_SM = 64
 # Algorithmic work per verification, the fixed roofline numerator: the
 # reference's operation count (gpu-crypto/cuda/api.cu:22-91 over
@@ -61,8 +63,8 @@ ALGO_FP_MULS_PER_VERIFY = 16941
 IMAD_PER_FP_MUL = 588   # the reference CIOS multiply: 12 rows x (24 for a b_i + 1 for m + 24 for m p)
 ALGO_IMAD_PER_VERIFY = ALGO_FP_MULS_PER_VERIFY * IMAD_PER_FP_MUL
 # DRAM bytes of one 4,096-verify launch of the verify kernel (k_verify_w),
-# measured with ncu (1.76 MB read, 0 written): the kernel is not memory-bound.
-DRAM_BYTES_PER_LAUNCH = 1762560
+# measured with ncu (1.71 MB read, 0 written): the kernel is not memory-bound.
+DRAM_BYTES_PER_LAUNCH = 1712128
 
 
 def dist_env():
@@ -422,20 +424,22 @@ def run_gpu(args):
         clk = clocks["sm_mhz"] or float(load_peaks().get("sm_max_mhz", 1965.0))
         peak_timad = sms * IMAD_PER_CLK_PER_SM * clk * 1e6 / 1e12
         achieved_timad = ALGO_IMAD_PER_VERIFY * N_ITEMS / (kernel_ms / 1e3) / 1e12
+        kernel = (("k_verify_fp2" if args.threads_per_block == 64 else "k_verify_w") if args.lanes == 6
+                  else "k_verify_lanes<%d>" % args.lanes) if args.lanes > 1 else "k_verify"
+        own = OWN_WORK.get(kernel)
+        traffic = DRAM_BYTES_PER_LAUNCH if kernel == "k_verify_w" else None
         roofline = {
             "bound": "int32-imad", "achieved": round(achieved_timad, 3), "peak": round(peak_timad, 3),
-            "unit": "TIMAD/s", "frac": round(achieved_timad / peak_timad, 4), "traffic": DRAM_BYTES_PER_LAUNCH,
+            "unit": "TIMAD/s", "frac": round(achieved_timad / peak_timad, 4), "traffic": traffic,
             "traffic_basis": "dram__bytes_read.sum + dram__bytes_write.sum of one 4,096-verify launch from an "
                              "ncu capture of this kernel (line tables and points; the bound is the IMAD pipe, "
                              "not DRAM)",
             "peak_basis": "%d SMs x 64 IMAD/clk x %.0f MHz (median SM clock sampled during the timed region)"
                           % (sms, clk),
             "algorithmic_imad_per_verify": ALGO_IMAD_PER_VERIFY,
-            "own_imad_per_verify": IMAD_PER_VERIFY, "own_products_per_verify": OWN_PRODUCTS_PER_VERIFY,
-            "own_reductions_per_verify": OWN_REDC_PER_VERIFY,
-            "kernel": (("k_verify_fp2" if args.threads_per_block == 64 else "k_verify_w") if args.lanes == 6
-                       else "k_verify_lanes<%d>" % args.lanes) if args.lanes > 1
-            else "k_verify",
+            "own_imad_per_verify": own[0] * 216 + own[1] * 300 if own else None,
+            "own_products_per_verify": own[0] if own else None, "own_reductions_per_verify": own[1] if own else None,
+            "kernel": kernel,
             "kernel_ms": round(kernel_ms, 4),
             "chain_ceiling": round(chain_timad, 3),
             "frac_of_chain_ceiling": round(achieved_timad / chain_timad, 4),
@@ -444,24 +448,16 @@ def run_gpu(args):
                                    "(bls_imad_chain_rate)",
             # The nominal peak counts every IMAD at the full rate, but only the
             # low-word multiply issues at that rate: the high word (mul.hi /
-            # mul.wide) is measured at half of it.  Separate low-word and
-            # high-word multiplies, half of each, retire at most at the harmonic
-            # mean of the two rates.  The kernels' products write both multiply-adds
-            # of a pair of limbs next to each other, which issue as one 64-bit
-            # multiply-add, so they can exceed that mean.
+            # mul.wide) is measured at half of it, and so is a pair of both on the
+            # same operands, which issues as one 64-bit multiply-add.
             "imad_lo_rate": round(lo_rate / 1e12, 3),
             "imad_hi_rate": round(hi_rate / 1e12, 3),
-            "mix_peak": round(2.0 / (1e12 / lo_rate + 1e12 / hi_rate), 3),
-            "frac_of_mix_peak": round(achieved_timad / (2.0 / (1e12 / lo_rate + 1e12 / hi_rate)), 4),
-            "mix_peak_basis": "measured (bls_imad_pipe_rates): independent mad.lo.u32 and mad.hi.u32 with every "
-                              "latency covered; separate low and high multiplies, half of each, retire at most at "
-                              "their harmonic mean; pairs of both on the same operands issue as one and can exceed it",
+            "imad_rates_basis": "measured (bls_imad_pipe_rates): independent mad.lo.u32 and mad.hi.u32 with every "
+                                "latency covered; a pair of both on the same operands issues at the high word's rate",
         }
         if full_chip:
             fc_timad = ALGO_IMAD_PER_VERIFY * full_chip["items"] / (full_chip["kernel_ms"] / 1e3) / 1e12
-            full_chip.update({"achieved": round(fc_timad, 3), "frac": round(fc_timad / peak_timad, 4),
-                              "frac_of_mix_peak": roofline["mix_peak"] and
-                              round(fc_timad / roofline["mix_peak"], 4)})
+            full_chip.update({"achieved": round(fc_timad, 3), "frac": round(fc_timad / peak_timad, 4)})
             roofline["full_chip"] = full_chip
         result = {
             "metric": METRIC, "value": round(value, 1), "unit": "verifies/s", "n_gpus": world,
