@@ -425,10 +425,18 @@ class Working {
 class Settled {
   public:
     explicit Settled(bls_ctx* c) : c_(c) {}
-    ~Settled() { cudaStreamSynchronize(c_->stream); }
+    ~Settled() {
+        if (!last_) cudaStreamSynchronize(c_->stream);
+    }
+    // the call's last wait: nothing is queued after it
+    cudaError_t wait() {
+        last_ = true;
+        return cudaStreamSynchronize(c_->stream);
+    }
 
   private:
     bls_ctx* c_;
+    bool last_ = false;
 };
 
 // What a verify of n items plans with: SMs for its decode, and lanes to an item (0
@@ -900,7 +908,7 @@ int bls_g2_decompress_status(bls_ctx* ctx, const uint8_t* in, int n, uint64_t* q
                                  nullptr, ctx->use.share(1), ctx->stream));
     CK(cudaMemcpyAsync(q24, ctx->d_xy.p, k * 192, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(status, ctx->d_st.p, k * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    CK(copies.wait());
     return BLS_OK;
 }
 
@@ -942,7 +950,7 @@ int bls_verify_batch(bls_ctx* ctx, const bls_batch* b, int32_t* results) {
         return rc;
     if (b->miller_out) CK(cudaMemcpyAsync(b->miller_out, ctx->d_ml.p, n * 576, cudaMemcpyDeviceToHost, ctx->stream));
     if (b->gt_out) CK(cudaMemcpyAsync(b->gt_out, ctx->d_gt.p, n * 576, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    CK(copies.wait());
     memcpy(results, ctx->h_res.p, n * 4);
     return BLS_OK;
 }
@@ -1027,7 +1035,7 @@ int bls_verify_requests(bls_ctx* ctx, const bls_request* reqs, int nreq, int fmt
         ctx->graph_key = key;
     }
     CK(cudaGraphLaunch(ctx->graph, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    CK(copies.wait());
     for (int r = 0; r < nreq; ++r)
         memcpy(reqs[r].results, (const char*)ctx->h_res.p + first[r] * 4, (size_t)reqs[r].n * 4);
     return BLS_OK;
@@ -1331,7 +1339,7 @@ int bls_neg_hash_to_g1(bls_ctx* ctx, const uint8_t* msgs, const uint32_t* offset
     Working call(ctx);
     if ((rc = stage_hash(ctx, msgs, offsets, n, dst, dst_len))) return rc;
     CK(cudaMemcpyAsync(out, ctx->d_nhms.p, (size_t)n * 96, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    CK(copies.wait());
     return BLS_OK;
 }
 
@@ -1357,7 +1365,7 @@ int bls_verify_messages(bls_ctx* ctx, int fmt, const void* sigs, const uint8_t* 
     const bool decode = fmt == BLS_SIG_COMPRESSED && ctx->cfg.lanes_per_pairing != 1;
     if ((rc = stage_hash(ctx, msgs, offsets, n, dst, dst_len, decode))) return rc;
     if ((rc = enqueue(ctx, k, fmt, false, false, false, true, true, decode))) return rc;
-    CK(cudaStreamSynchronize(ctx->stream));
+    CK(copies.wait());
     memcpy(results, ctx->h_res.p, k * 4);
     return BLS_OK;
 }
@@ -1379,7 +1387,7 @@ int bls_g1_decompress_status(bls_ctx* ctx, const uint8_t* in, int n, uint64_t* x
                                  ctx->use.share(1), ctx->stream));
     CK(cudaMemcpyAsync(xy, ctx->d_xy.p, (size_t)n * 96, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(status, ctx->d_st.p, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    CK(copies.wait());
     return BLS_OK;
 }
 
