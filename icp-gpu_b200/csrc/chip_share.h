@@ -2,10 +2,11 @@
 //
 // The forms with several lanes to an item (verify_w.cu, g1.cuh, h2c.cuh, g2.cuh) buy a
 // small batch latency with SM time: a block of the 32-item kernel fills an SM, and 32
-// items on four lanes each hold 4 SMs for 2.51 ms where a lane each holds one for 3.47,
+// items on four lanes each hold 4 SMs for 2.49 ms where a lane each holds one for 3.42,
 // 2.9 times as much.  That is right while the SMs would stand idle, and wrong when other
 // launches would have run on them: three launches of 1,184 items are 37 blocks each and
-// run side by side with a lane an item, but fill the chip three times over with four.
+// run side by side with a lane an item, but fill the chip three times over with four
+// (together 3.48 and 7.48 ms; 8 x 300 items 3.50 and 7.44).
 // So every call that launches such a kernel is counted on its device from where it
 // starts to where its work has run, with the SMs that its verify launch holds, and a
 // launch plans with the SMs the others leave.  Only the time depends on it: every

@@ -23,9 +23,9 @@
 // What it is bound by: a paired multiply-add holds the multiply pipe as long as
 // mul.hi alone does (4 cycles a warp and scheduler), and mul.lo half of that, so
 // rows of separate mul.lo and mul.hi chains cost 6 cycles a limb product where
-// the pair costs 4.  Twelve warps on each of 148 SMs, one dependent product after
-// another: 30.3 G products/s, 97% of the pair's issue rate, against 18.8 G with
-// separate rows; one warp alone, 951 ns a product against 1,292 ns.
+// the pair costs 4.  The paired columns made every workload 1.24 to 1.52 times as
+// fast; the 12 x 12-limb product alone, operands from shared memory, went from 41.4
+// to 57.3 G products/s on 148 SMs (bls_limb_layout_rates).
 //
 // This replaces the reference's vendored sppark fp_t (gpu-crypto/cuda/vendor/
 // sppark/mont_t.cuh:381-422, constants bls12-381.hpp:13-33) and is written from

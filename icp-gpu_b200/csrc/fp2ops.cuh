@@ -154,9 +154,8 @@ __device__ __forceinline__ void prod24(uint32_t* p, const uint32_t* a, const uin
 // p = L + (M - L - H) 2^192 + H 2^384.  Three 6 x 6 products (108 paired
 // multiply-adds) instead of 144; the sums and corrections are plain adds, on
 // the pipe that the multiplies leave free.  Twelve warps an SM, operands from
-// shared memory and the product accumulated: 56.5 G products/s on 148 SMs,
-// against 54.8 G for the schoolbook product in the same pairs and 42.0 G for
-// this Karatsuba over separate mul.lo and mul.hi rows.
+// shared memory and the product accumulated: 57.3 G products/s on 148 SMs
+// (bls_limb_layout_rates), against 41.4 G over separate mul.lo and mul.hi rows.
 __device__ __forceinline__ void prod24k(uint32_t* p, const uint32_t* a, const uint32_t* b) {
     uint32_t sa[6], sb[6], ca, cb;
     asm("add.cc.u32 %0, %7, %13;\n\t"
@@ -647,8 +646,8 @@ __device__ __forceinline__ void add12(uint32_t* r, const uint32_t* a, const uint
         : BLS_A12(a), BLS_A12(b));
 }
 
-// x = 3p - x and x = 5p - x (12 limbs), the multiples as immediates (read from
-// constant memory: 3.79 against 3.75 ms per 4,096 verifications)
+// x = 3p - x and x = 5p - x (12 limbs), the multiples as immediates (reading them
+// from constant memory is slower)
 __device__ __forceinline__ void sub_from_3p(uint32_t* x) {
     asm("sub.cc.u32 %0, 0xffff0001, %0;\n\t"
         "subc.cc.u32 %1, 0x2dfcffff, %1;\n\t"

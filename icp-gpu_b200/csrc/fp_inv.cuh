@@ -1,5 +1,7 @@
 // Fp inverse by Bernstein and Yang's division steps ("Fast constant-time gcd
-// computation and modular inversion", CHES 2019), shared by the verify kernels
+// computation and modular inversion", CHES 2019), counting delta in halves and in
+// thirty-bit limbs as in the public description of libsecp256k1's inverse (Dettman,
+// Wuille: doc/safegcd_implementation.md of that project), shared by the verify kernels
 // (the final exponentiation's one inversion), the line tables and the hash to G1.
 //
 // One step takes (delta, f, g), f odd, to
@@ -14,10 +16,10 @@
 // Values are signed, in thirteen limbs of thirty bits, so that a limb product is
 // one signed wide multiply-add and there are no carry chains.  Nothing branches
 // on the value but the end of the loop (26 or 27 rounds for 381 bits), so the
-// lanes of a warp invert different values side by side: 67 k cycles (34 us) a
-// warp, bound by one warp's dependent chain.  A binary Euclid diverges; on the
-// product of the warp's values (prefix and suffix products by shuffles), which
-// avoids that, it took 287 k cycles, and the verify kernel 3.60 instead of 3.50 ms.
+// lanes of a warp invert different values side by side, bound by one warp's
+// dependent chain.  A binary Euclid diverges; with one on the product of the warp's
+// values (prefix and suffix products by shuffles), which avoids that, the verify
+// kernel took 3.60 instead of 3.50 ms.
 #pragma once
 #include "fp.cuh"
 
@@ -25,8 +27,9 @@ namespace bls {
 
 constexpr int kInvLimbs = 13, kInvBits = 30;
 constexpr int32_t kInvMask = (1 << kInvBits) - 1;
-// (49 * 381 + 57) / 17 = 1,101 steps suffice from delta = 1, fewer from 1/2
-// (Theorem 11.2 there); the loop ends when g is zero
+// Theorem 11.2 of the paper: (49 * 381 + 57) / 17 = 1,101 steps suffice from delta = 1
+// (741 for 256 bits).  From 1/2 fewer do: 590 for 256 bits in the description named
+// above.  The loop ends when g is zero, after at most 1,110 steps.
 constexpr int kInvMaxRounds = 37;
 
 __device__ __forceinline__ void inv_limbs(int32_t* r, const uint32_t* w) {

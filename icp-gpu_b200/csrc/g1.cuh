@@ -175,9 +175,7 @@ __device__ __forceinline__ fp fp_sel(bool c, const fp& a, const fp& b) {
 
 // dbl-2009-l, with Z3 = (Y + Z)^2 - Y^2 - Z^2 to make its first level four squares
 // and (2B)^2 beside B^2 in the second; sums that are squared or multiplied next
-// are left unreduced (fp_sqr takes values below 3p).  A lone warp's doubling is
-// then 4,760 cycles of two squares and a product, 900 of additions and 300 of
-// shuffles, against 12,500 for one lane a point.
+// are left unreduced (fp_sqr takes values below 3p).
 __device__ __forceinline__ g1j quad_dbl(const g1j& p) {
     const int l = threadIdx.x & 3;
     fp s = fp_sqr(fp_sel(l < 2, fp_sel(l == 0, p.X, p.Y), fp_sel(l == 2, fp_add_nr(p.Y, p.Z), p.Z)));

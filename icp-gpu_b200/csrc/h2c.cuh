@@ -48,9 +48,8 @@ static __device__ __noinline__ void sha256_block(uint32_t* h, const uint32_t* bl
 
 // The hash state after `bytes` bytes of a stream whose byte p is at(p) for p < len,
 // the first `done` of them in h already (a multiple of 64): the rest, the padding
-// and the length.  Blocks are put together a word at a time; fed byte by byte
-// through a buffer in local memory, a 32-byte message's expansion took 229 k
-// cycles, a seventh of its whole hash, against 101 k.
+// and the length.  Blocks are put together a word at a time, not fed byte by byte
+// through a buffer in local memory.
 template <class At>
 __device__ __forceinline__ void sha256_finish(uint32_t* h, uint32_t done, uint64_t len, At at) {
     const uint64_t blocks = (len + 8) / 64 + 1;

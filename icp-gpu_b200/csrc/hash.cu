@@ -94,9 +94,8 @@ __global__ void __launch_bounds__(kHashThreads) k_neg_hash_decode_wide(const uin
 // together (the power is a chain that all four repeat), evaluate one polynomial of
 // the isogeny each, and the two quads exchange their points and clear the cofactor
 // with the products of a level side by side (quad_add, quad_dbl).
-// Bound by one dependent chain, for a 32-byte message in cycles: expansion 101 k,
-// the map with its power of 379 squarings 818 k, isogeny 108 k, sum and cofactor
-// 479 k, inverse 78 k.
+// Bound by one dependent chain, half of it the map's power of 379 squarings, most of the
+// rest the sum and the cofactor's 63 doublings.
 __device__ __forceinline__ void neg_hash_quad(int t, const uint8_t* msgs, const uint32_t* offsets, int n,
                                               const uint8_t* dst, int dst_len, uint64_t* out) {
     const int which = (t >> 2) & 1;

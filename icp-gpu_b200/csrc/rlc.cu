@@ -90,8 +90,8 @@ static __device__ __noinline__ bool g1_point_ok(const fp& x, const fp& y) {
 // (0: [r] sig, 1: [r] nhm, 2: sig checks, 3: nhm checks), so a warp never
 // splits between the scalar multiplication and the checks.  Bound by the multiply
 // pipe and its carries; four blocks an SM (128 registers) instead of two: 16,384
-// items 2.89 -> 2.37 ms.  (The roles moved on by one warp from block to block,
-// which evens the schedulers out, 2.63 ms.)
+// items 2.89 -> 2.37 ms.  (The roles moved on by one warp from block to block evens
+// the schedulers out and is slower.)
 __global__ void __launch_bounds__(128, 4) k_rlc_scale(const uint64_t* sig_xy, const int32_t* status,
                                                    const uint64_t* nhms, const uint64_t* r, int n, int check_sig,
                                                    uint32_t* pts, uint8_t* bad, int* counters) {

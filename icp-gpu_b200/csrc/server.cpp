@@ -143,7 +143,7 @@ constexpr int32_t kSentinel = 0x7fffffff;
 // flight) takes at most kDecSmsPerRound SMs, so the decoder never holds more
 // than the SMs set aside for it and the ring kernel's blocks always find
 // theirs.  The four rounds keep up with the other 136 SMs' verifies (about 9 k/s
-// per SM): 1.235 M verifies/s saturated, against 1.355 M for points that need
+// per SM): 1.25 M verifies/s saturated, against 1.375 M for points that need
 // no decode on all 148.
 constexpr int kDecSmsPerRound = 3;
 constexpr int kDecodeSms = Ring::kDecStreams * kDecSmsPerRound;

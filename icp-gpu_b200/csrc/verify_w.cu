@@ -19,10 +19,10 @@
 // counts.  Against the form in which the two warps of a coefficient each added
 // every product into two accumulators (verify_fp2.cu's): one accumulator, no bias
 // to preload, one range reduction per component instead of two: 3.92 -> 3.60 ms
-// per 4,096 verifications.  Also measured, and slower: one warp a component with
-// no partial sums and a third more products, accumulated in place (4.34 ms);
-// eighteen warps, three to a coefficient, at the 96 registers that leaves (4.33 ms,
-// spills); operands of the next product loaded ahead (3.90 against 3.79 ms).
+// per 4,096 verifications (3.42 with what came after it).  Also measured, and
+// slower: one warp a component with no partial sums and a third more products,
+// accumulated in place; eighteen warps, three to a coefficient, at the 96 registers
+// that leaves; operands of the next product loaded ahead.
 //
 // Shared memory (16-byte units): the items' Fp2 slots interleaved by item
 // (unit ((s * 2 + c) * 3 + q) * 32 + v holds words 4q..4q+3 of component c of
@@ -143,8 +143,7 @@ __device__ __forceinline__ void load_form(uint32_t* x, const Sm& s, uint32_t f, 
 
 // The operands U, V of the product described by w (gen_fp2ops.py: COMBOS).  The
 // pairs of forms that the hot programs use have a case each, with all loads
-// ahead of the arithmetic (two calls of load_form cost a lone warp 580 cycles a
-// product, these cases 380; 3.65 -> 3.60 ms).
+// ahead of the arithmetic, where two calls of load_form wait for each of theirs.
 __device__ __forceinline__ void load_operands(uint32_t* U, uint32_t* V, const Sm& s, uint32_t w, const Bases& bs,
                                               const uint32_t* line) {
     const uint32_t xs = slot_addr(bs, (w >> 8) & 0x7fu), ys = slot_addr(bs, (w >> 16) & 0x7fu);
@@ -518,7 +517,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_verify_w(VerifyArgs a, const ui
     s.flags = reinterpret_cast<uint8_t*>(s.info + kInfoWords);
     s.bcast = reinterpret_cast<uint32_t*>(s.flags + kFlagBytes);
     // from a shuffle, so that the compiler knows it to be uniform in the warp:
-    // descriptor decoding and branches on uniform registers (3.75 -> 3.65 ms)
+    // descriptor decoding and branches on uniform registers
     const int role = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
     const int half = role / 6, k = role % 6;
     s.v = threadIdx.x & (kItems - 1);
@@ -745,11 +744,11 @@ VerifyArgs items_from(VerifyArgs a, int first) {
 
 // As many lanes to an item as still give every item a place in one wave of the SMs that
 // the launch plans with (chip_share.h): four up to 8 items a SM, two up to 16.  One
-// launch alone of a block on every SM takes 3.47 ms with a lane to an item, 2.77 ms with
-// two and 2.51 ms with four (the sums shrink from 2, 3, 5 and 9 products in the
+// launch alone of a block on every SM takes 3.42 ms with a lane to an item, 2.74 ms with
+// two and 2.49 ms with four (the sums shrink from 2, 3, 5 and 9 products in the
 // cyclotomic square, the line, the square and the product to 1, 2, 3 and 5, or 1, 1, 2
 // and 3; the reductions stay).  A batch of several waves whose last one would be that
-// empty runs it as a launch of its own: 4,737 items 7.0 -> 6.0 ms.
+// empty runs it as a launch of its own: 4,737 items 5.91 ms, against 6.84 for two whole waves.
 cudaError_t launch_verify_w(const VerifyArgs& a, const uint32_t* in_status, int sms, cudaStream_t s) {
     if (a.n <= 0) return cudaSuccess;
     cudaError_t e = configure();
