@@ -43,17 +43,21 @@ class ChipUse {
     ChipUse& operator=(const ChipUse&) = delete;
     ~ChipUse() { end(); }
 
-    void begin(int device, int sms) {
+    // caller: a call of a context; false for a server's launches, which come from a queue
+    // that the server sees, and tell nothing about how many callers there will be
+    void begin(int device, int sms, bool caller = true) {
+        end();
         Chip& c = chip(device);
         std::lock_guard<std::mutex> lk(c.mu);
-        if (on_) leave(*chip_);
         reap(c);
         chip_ = &c;
         sms_ = sms;
         on_ = waiting_ = true;
         next_ = c.uses;
         c.uses = this;
-        c.peak = std::max(c.peak, ++c.users);
+        caller_ = caller;
+        ++c.users;
+        if (caller) c.peak = std::max(c.peak, ++c.callers);
     }
     void end() {
         if (!chip_) return;
@@ -71,7 +75,7 @@ class ChipUse {
 
     // SMs a launch that needs at least `need` of them plans with: of those that no
     // other use holds an equal part, the uses that have not launched yet having theirs to
-    // come.  expect: as many uses are expected as met in the last busy time of the device
+    // come.  expect: as many callers are expected as met the last time there were any
     // (calls that return before their work is done show up one after another; a server
     // knows its own queue).  Where the part is too small the launch has to wait for others
     // in any case, and plans with an equal part of the whole chip, of which the uses that
@@ -101,8 +105,8 @@ class ChipUse {
     struct Chip {
         std::mutex mu;
         ChipUse* uses = nullptr;       // begun and not ended, linked by next_
-        int users = 0;                 // how many
-        int peak = 0, last_peak = 0;   // most at once: since the device was last idle, and before
+        int users = 0, callers = 0;    // how many, and of those, calls of contexts
+        int peak = 0, last_peak = 0;   // most callers at once: since there was none, and before
     };
     static constexpr int kChips = 64;
     static Chip& chip(int device) {
@@ -112,7 +116,7 @@ class ChipUse {
 
     int share_locked(int need, bool expect) const {
         const Chip& c = *chip_;
-        const int missing = expect ? std::max(0, c.last_peak - c.users) : 0;
+        const int missing = expect ? std::max(0, c.last_peak - c.callers) : 0;
         int held = 0, waiting = 0;
         for (const ChipUse* u = c.uses; u; u = u->next_) {
             if (u == this) continue;
@@ -141,7 +145,8 @@ class ChipUse {
         ChipUse** at = &c.uses;
         while (*at != this) at = &(*at)->next_;
         *at = next_;
-        if (--c.users == 0) {
+        --c.users;
+        if (caller_ && --c.callers == 0) {
             c.last_peak = c.peak;
             c.peak = 0;
         }
@@ -158,7 +163,7 @@ class ChipUse {
 
     Chip* chip_ = nullptr;
     int sms_ = 0, held_ = 0;
-    bool on_ = false, waiting_ = false;
+    bool on_ = false, waiting_ = false, caller_ = false;
     bool (*done_)(const void*) = nullptr;
     const void* what_ = nullptr;
     ChipUse* next_ = nullptr;

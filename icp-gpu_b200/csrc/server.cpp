@@ -176,7 +176,7 @@ struct bls_server {
             n += r.n;
         }
         cudaStream_t st = s.stream;
-        s.use.begin(view.device, view.sms);
+        s.use.begin(view.device, view.sms, false);
         if (cudaMemcpyAsync(s.d_sigs, s.h_sigs, n * sb, cudaMemcpyHostToDevice, st) ||
             cudaMemcpyAsync(s.d_nhms, s.h_nhms, n * 96, cudaMemcpyHostToDevice, st) ||
             cudaMemcpyAsync(s.d_ids, s.h_ids, n * 4, cudaMemcpyHostToDevice, st) ||
@@ -262,7 +262,7 @@ struct bls_server {
                                   ? bls::launch_verify_w_serve(a, st, blocks, view.sms, ring.kern)
                                   : bls::launch_verify_fp2_serve(a, st, blocks, view.sms, ring.kern);
         if (e != cudaSuccess || cudaEventRecord(ring.done, ring.kern) != cudaSuccess) return BLS_ERR_CUDA;
-        ring.use.begin(view.device, view.sms);
+        ring.use.begin(view.device, view.sms, false);
         if (view.shape == bls::kShapeWide) ring.use.hold(blocks < view.sms ? blocks : view.sms);
         ring.use.end_when(bls::event_done, ring.done);
         ring.launched = true;

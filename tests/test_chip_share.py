@@ -16,7 +16,7 @@ DRIVER = r"""
 #include <iostream>
 #include <string>
 #include "chip_share.h"
-// one command a line: b use device | p use n expect -> lanes | s use need expect -> share |
+// one command a line: b use device (B: a server's) | p use n expect -> lanes | s use need expect -> share |
 // h use sms | w use (ends when its flag is up) | f use (its flag) | e use
 int main() {
     static bls::ChipUse uses[8];
@@ -24,7 +24,7 @@ int main() {
     std::string op;
     int u, a, x;
     while (std::cin >> op >> u) {
-        if (op == "b") { std::cin >> a; flag[u] = false; uses[u].begin(a, 148); }
+        if (op == "b" || op == "B") { std::cin >> a; flag[u] = false; uses[u].begin(a, 148, op == "b"); }
         if (op == "p") { std::cin >> a >> x; std::cout << uses[u].plan_verify(a, x != 0) << "\n"; }
         if (op == "s") { std::cin >> a >> x; std::cout << uses[u].share(a, x != 0) << "\n"; }
         if (op == "h") { std::cin >> a; uses[u].hold(a); }
@@ -90,18 +90,24 @@ def test_calls_that_return_early_are_expected_again(plan):
 
 def test_a_server_knows_its_own_queue(plan):
     """slots: the first requests of a burst, then the bulk, which no one follows"""
-    first = ["b 0 0", "p 0 10 0", "b 1 0", "p 1 20 0", "b 2 0", "p 2 1000 0"]
-    assert plan(first + ["e 0", "e 1", "e 2"] + first) == [4, 4, 4] * 2
-    full = ["b 0 0", f"p 0 {8 * SMS} 0", "b 1 0", f"p 1 {8 * SMS} 0", "b 2 0", f"p 2 {8 * SMS} 0"]
-    refill = ["e 0", "b 0 0", f"p 0 {8 * SMS} 0", "e 1", "b 1 0", f"p 1 {8 * SMS} 0", "e 2", "b 2 0", f"p 2 {8 * SMS} 0"]
+    first = ["B 0 0", "p 0 10 0", "B 1 0", "p 1 20 0", "B 2 0", "p 2 1000 0"]
+    done = ["e 0", "e 1", "e 2"]
+    assert plan(first + done + first) == [4, 4, 4] * 2
+    # and does not make a context that calls alone afterwards, or beside it, hold back
+    assert plan((first + done + ["b 3 0", f"p 3 {8 * SMS} 1", "e 3"]) * 2) == [4, 4, 4, 4] * 2
+    full = ["B 0 0", f"p 0 {8 * SMS} 0", "B 1 0", f"p 1 {8 * SMS} 0", "B 2 0", f"p 2 {8 * SMS} 0"]
+    refill = ["e 0", "B 0 0", f"p 0 {8 * SMS} 0", "e 1", "B 1 0", f"p 1 {8 * SMS} 0", "e 2", "B 2 0", f"p 2 {8 * SMS} 0"]
     got = plan(full + refill * 3)
     for k in range(3, len(got) - 2, 3):
         assert sum(held(8 * SMS, lanes) for lanes in got[k:k + 3]) <= SMS
 
 
 def test_a_resident_kernel_leaves_the_rest(plan):
-    assert plan(["b 7 0", "h 7 136", "w 7", "b 0 0", "p 0 300 1", "e 0", "f 7", "b 0 0", "p 0 300 1", "b 0 0", "p 0 300 1"]) \
+    assert plan(["B 7 0", "h 7 136", "w 7", "b 0 0", "p 0 300 1", "e 0", "f 7", "b 0 0", "p 0 300 1", "b 0 0", "p 0 300 1"]) \
         == [1, 4, 4]
+    # while it stays, callers that met once are not expected for ever
+    three = ["b 0 0", "b 1 0", "b 2 0", "e 0", "e 1", "e 2"]
+    assert plan(["B 7 0", "h 7 12", "w 7"] + three + ["b 0 0", "p 0 1000 1", "e 0"] * 3) == [1, 4, 4]
 
 
 def test_nothing_stays_counted(plan):
@@ -111,7 +117,7 @@ def test_nothing_stays_counted(plan):
     for _ in range(3000):
         u = rng.randrange(1, 8)
         if state[u] == "off":
-            script.append(f"b {u} 0")
+            script.append(rng.choice([f"b {u} 0", f"B {u} 0"]))
             state[u] = "on"
         elif state[u] == "on":
             script.append(rng.choice([f"p {u} {rng.randrange(1, 20000)} {rng.randrange(2)}", f"s {u} 5 1", f"h {u} 7", f"e {u}", f"w {u}"]))
